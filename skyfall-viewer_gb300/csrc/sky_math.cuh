@@ -81,6 +81,39 @@ SKY_DEV float sky_expf_inrange(float x) {
   return __uint_as_float(__float_as_uint(p) + (kbits << 23));
 }
 
+// Products of packed f32x2 operations that are rounded before they are added
+// to something: the assembler contracts a packed multiply and a packed add
+// into a fused multiply-add whatever the rounding modifiers and -fmad say
+// (checked: 26 % of random a * b + c differ from the two roundings), and it
+// folds an addend it knows to be -0.  neg_zero is -0.0f from a kernel
+// parameter: x y + (-0) is the rounded product bit for bit, signs of zero
+// included, at the same rate as the multiply.
+SKY_DEV float2 mul2_rounded(float2 x, float2 y, float neg_zero) {
+  return __ffma2_rn(x, y, make_float2(neg_zero, neg_zero));
+}
+
+// sky_expf_inrange(-s) of two arguments in packed f32x2 operations: the same
+// operations in the same order, with the reduced argument's sign turned (r =
+// -r', a rounding is symmetric in sign) so that neither s nor k has to be
+// negated.  2^k is added through the exponent field: the rounding constant's
+// own bits shift out.
+SKY_DEV float2 sky_expf_neg_pair(float2 s, float neg_zero) {
+  auto c2 = [](float v) { return make_float2(v, v); };
+  const float2 u = __fadd2_rn(mul2_rounded(s, c2(-1.44269502f), neg_zero), c2(12582912.0f));
+  const float2 k = __fadd2_rn(u, c2(-12582912.0f));
+  float2 r = __ffma2_rn(k, c2(0.693147182f), s);
+  r = __ffma2_rn(k, c2(-1.90465421e-09f), r);
+  float2 p = __ffma2_rn(c2(-1.98412701e-04f), r, c2(1.38888892e-03f));
+  p = __ffma2_rn(p, r, c2(-8.33333377e-03f));
+  p = __ffma2_rn(p, r, c2(4.16666679e-02f));
+  p = __ffma2_rn(p, r, c2(-1.66666672e-01f));
+  p = __ffma2_rn(p, r, c2(0.5f));
+  p = __ffma2_rn(p, r, c2(-1.0f));
+  p = __ffma2_rn(p, r, c2(1.0f));
+  return make_float2(__uint_as_float(__float_as_uint(p.x) + (__float_as_uint(u.x) << 23)),
+                     __uint_as_float(__float_as_uint(p.y) + (__float_as_uint(u.y) << 23)));
+}
+
 // log(x): x = m 2^e with m in [sqrt(1/2), sqrt(2)); log m = 2 atanh(s),
 // s = (m - 1) / (m + 1), |s| <= 0.172, by its odd series to s^11 (Horner in
 // s^2, fused multiply-adds); log x = e ln2 + log m with ln2 split in two.

@@ -232,46 +232,125 @@ __global__ void k_viewer_ranges(const uint32_t* __restrict__ keys, uint32_t tota
 
 constexpr int kViewBatch = 256;
 
-__global__ void __launch_bounds__(kViewTile* kViewTile)
+// Two splats of a warp's list side by side, so that a lane evaluates both with
+// packed operations: each float2 holds the first and the second splat's value.
+struct __align__(16) SplatPair {
+  float2 nmx, nmy;     // negated means
+  float2 a, c;         // conic
+  float2 b, opacity;
+  float2 bits, blue;   // coverage bits, blue
+  float2 rg[2];        // red and green of either splat
+};
+
+// One CTA per 16x16 tile, warp w on its 8x4 pixel block (w & 1, w >> 1).  The
+// thread that stages a splat runs the quad's coverage test once per pixel
+// column (low half of a word) and row (high half) of the tile; each warp
+// lists the splats with a column and a row in its block and blends them in
+// order, a pixel's test being its two bits.  The list is walked two splats at
+// a time, copied side by side into shared memory 32 entries ahead (one per
+// lane): exponents and exponentials are packed f32x2 operations, the blends
+// follow in order.  Issue-bound: every covered (pixel, splat) pair has to be
+// blended, back to front, with no early exit.  1M Gaussians at 1920x1080:
+// 2184 us with warps that tested every quad of the tile at every pixel, 1595
+// with lists and coverage bits, 1276 with pairs.
+__global__ void __launch_bounds__(kViewTile* kViewTile, 5)
 k_viewer_raster(ViewerParams vp, const float4* __restrict__ splats,
                 const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ gidx,
                 float4* __restrict__ rgba) {
-  __shared__ float4 s_sp[kViewBatch * 3];
+  constexpr int NT = kViewTile * kViewTile;
+  static_assert(kViewTile == 16 && kViewBatch == NT, "16-bit masks; one staged splat per thread");
+  __shared__ float4 s_sp[kViewBatch][2];   // mean, conic a, b | conic c, opacity, red, green
+  __shared__ float2 s_bc[kViewBatch];      // blue, coverage bits
+  __shared__ uint8_t s_list[NT / 32][kViewBatch];
+  __shared__ SplatPair s_pair[NT / 32][16];
   const uint32_t tile = blockIdx.x;
   const uint32_t tx = tile % vp.tiles_x, ty = tile / vp.tiles_x;
-  const uint32_t tid = threadIdx.x;
-  const uint32_t x = tx * kViewTile + tid % kViewTile, y = ty * kViewTile + tid / kViewTile;
+  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t lx = 8u * (warp & 1u) + (lane & 7u), ly = 4u * (warp >> 1) + (lane >> 3);
+  const uint32_t x = tx * kViewTile + lx, y = ty * kViewTile + ly;
   const bool inside = x < vp.width && y < vp.height;
-  const float pxf = (float)x + 0.5f, pyf = (float)y + 0.5f;
+  const float2 px2 = make_float2((float)x + 0.5f, (float)x + 0.5f);
+  const float2 py2 = make_float2((float)y + 0.5f, (float)y + 0.5f);
+  const uint32_t block_cols = 0xFFu << (8u * (warp & 1u));
+  const uint32_t block_rows = 0xF0000u << (4u * (warp >> 1));
+  const uint32_t my_bits = (1u << lx) | (0x10000u << ly);
+  const uint32_t lt = (1u << lane) - 1u;
   const uint32_t start = offsets[tile], end = offsets[tile + 1];
   float C0 = 0.0f, C1 = 0.0f, C2 = 0.0f, A = 0.0f;  // cleared to transparent black
   for (uint32_t bs = start; bs < end; bs += kViewBatch) {
     const uint32_t cnt = min((uint32_t)kViewBatch, end - bs);
     __syncthreads();
-    for (uint32_t k = tid; k < cnt; k += kViewTile * kViewTile) {
-      const size_t g = gidx[bs + k];
-      s_sp[k * 3 + 0] = splats[g * 3 + 0];
-      s_sp[k * 3 + 1] = splats[g * 3 + 1];
-      s_sp[k * 3 + 2] = splats[g * 3 + 2];
+    if (tid < cnt) {
+      const size_t g = gidx[bs + tid];
+      const float4 q0 = splats[g * 3 + 0], q2 = splats[g * 3 + 2];
+      s_sp[tid][1] = splats[g * 3 + 1];
+      s_sp[tid][0] = q0;
+      const float r = q2.y;
+      const float X0 = q0.x - r, X1 = q0.x + r, Y0 = q0.y - r, Y1 = q0.y + r;
+      uint32_t bits = 0u;
+#pragma unroll 4
+      for (uint32_t k = 0; k < (uint32_t)kViewTile; ++k) {
+        const float cx = (float)(tx * kViewTile + k) + 0.5f, cy = (float)(ty * kViewTile + k) + 0.5f;
+        if (cx >= X0 && cx < X1) bits |= 1u << k;
+        if (cy >= Y0 && cy < Y1) bits |= 0x10000u << k;
+      }
+      s_bc[tid] = make_float2(q2.x, __uint_as_float(bits));
     }
     __syncthreads();
-    if (!inside) continue;
-    for (uint32_t k = 0; k < cnt; ++k) {
-      const float4 q0 = s_sp[k * 3 + 0];
-      const float4 q2 = s_sp[k * 3 + 2];
-      const float r = q2.y;
-      if (!(pxf >= q0.x - r && pxf < q0.x + r && pyf >= q0.y - r && pyf < q0.y + r)) continue;
-      const float4 q1 = s_sp[k * 3 + 1];
-      const float dx = pxf - q0.x, dy = pyf - q0.y;
-      float s = 0.5f * ((q0.z * dx) * dx + (q1.x * dy) * dy);
-      s = s + (q0.w * dx) * dy;
-      if (s < 0.0f) continue;  // discard
-      const float a = clampf_(q1.y * sky_expf(-s), 0.0f, 1.0f);
-      const float om = 1.0f - a;
-      C0 = q1.z * a + C0 * om;
-      C1 = q1.w * a + C1 * om;
-      C2 = q2.x * a + C2 * om;
-      A = a + A * om;
+    uint32_t nlist = 0;
+    for (uint32_t base = 0; base < cnt; base += 32) {
+      const uint32_t j = base + lane;
+      const uint32_t bits = j < cnt ? __float_as_uint(s_bc[j].y) : 0u;
+      const bool in = (bits & block_cols) != 0u && (bits & block_rows) != 0u;
+      const uint32_t m = __ballot_sync(0xFFFFFFFFu, in);
+      if (in) s_list[warp][nlist + __popc(m & lt)] = (uint8_t)j;
+      nlist += __popc(m);
+    }
+    for (uint32_t base = 0; base < nlist; base += 32) {
+      __syncwarp();  // the list is written; the pairs before have been read
+      {
+        float* dst = reinterpret_cast<float*>(&s_pair[warp][lane >> 1]) + (lane & 1u);
+        if (base + lane < nlist) {
+          const uint32_t k = s_list[warp][base + lane];
+          const float4 q0 = s_sp[k][0], q1 = s_sp[k][1];
+          const float2 bc = s_bc[k];
+          dst[0] = -q0.x; dst[2] = -q0.y; dst[4] = q0.z; dst[6] = q1.x;
+          dst[8] = q0.w; dst[10] = q1.y; dst[12] = bc.y; dst[14] = bc.x;
+          s_pair[warp][lane >> 1].rg[lane & 1u] = make_float2(q1.z, q1.w);
+        } else {
+          dst[12] = 0.0f;  // covers nothing
+        }
+      }
+      __syncwarp();
+      const uint32_t np = (min(32u, nlist - base) + 1u) / 2u;
+      for (uint32_t p = 0; p < np; ++p) {
+        const SplatPair& q = s_pair[warp][p];
+        const float2 bits = q.bits;
+        const bool in0 = (~__float_as_uint(bits.x) & my_bits) == 0u;
+        const bool in1 = (~__float_as_uint(bits.y) & my_bits) == 0u;
+        if (!in0 && !in1) continue;  // outside both quads
+        const float2 dx = __fadd2_rn(px2, q.nmx), dy = __fadd2_rn(py2, q.nmy);
+        const float nz = vp.neg_zero;
+        const float2 s1 = mul2_rounded(__fmul2_rn(q.a, dx), dx, nz);
+        const float2 s2 = mul2_rounded(__fmul2_rn(q.c, dy), dy, nz);
+        float2 s = mul2_rounded(make_float2(0.5f, 0.5f), __fadd2_rn(s1, s2), nz);
+        s = __fadd2_rn(s, mul2_rounded(__fmul2_rn(q.b, dx), dy, nz));
+        float2 G = sky_expf_neg_pair(s, nz);
+        // (beyond the exponential's range, and NaN)
+        if (!(s.x <= 87.0f)) G.x = s.x != s.x ? s.x : 0.0f;
+        if (!(s.y <= 87.0f)) G.y = s.y != s.y ? s.y : 0.0f;
+        const float2 al = __fmul2_rn(q.opacity, G);
+        auto blend = [&](float a_raw, float2 rg, float blue) {
+          const float a = clampf_(a_raw, 0.0f, 1.0f);
+          const float om = 1.0f - a;
+          C0 = rg.x * a + C0 * om;
+          C1 = rg.y * a + C1 * om;
+          C2 = blue * a + C2 * om;
+          A = a + A * om;
+        };
+        if (in0 && !(s.x < 0.0f)) blend(al.x, q.rg[0], q.blue.x);
+        if (in1 && !(s.y < 0.0f)) blend(al.y, q.rg[1], q.blue.y);
+      }
     }
   }
   if (inside) rgba[(size_t)y * vp.width + x] = make_float4(C0, C1, C2, A);

@@ -18,6 +18,7 @@ struct ViewerParams {
   uint32_t round_f16;       // parameters read through f16 storage
   uint32_t n, plane_stride;
   uint32_t width, height, tiles_x, tiles_y;
+  float neg_zero = -0.0f;   // for mul2_rounded
 };
 
 // Per Gaussian: 3 float4 {cx, cy, a, b | c, opacity, r, g | b, radius, 0, 0},

@@ -1,0 +1,24 @@
+"""Viewer coverage at the edges of its 8x4 pixel blocks and 16x16 tiles, and
+lists longer than a staged batch: every (pixel, quad) pair and its order are
+the oracle's, so images are identical."""
+import numpy as np
+import pytest
+
+from skyfall import scenes
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("w,h,n,scaling", [(1, 1, 64, 1.0), (8, 4, 300, 1.0), (17, 16, 257, 2.0),
+                                           (33, 21, 3000, 1.0), (48, 48, 20000, 0.3)])
+def test_frame_matches_oracle_at_block_edges(sky, orc, w, h, n, scaling):
+    P = scenes.scene_uniform(n, seed=61)
+    P[3, ::7] = 0.5      # thin splats: exponents below the exp range inside the quad
+    P[4, ::7] = -6.0
+    P[10, ::5] = 20.0    # opacity 1
+    cam = scenes.camera_fov((0.1, -0.2, -2.0), w, h)
+    with sky.GaussianRenderer(sh_degree=0) as r:
+        r.load_points(P)
+        img = r.frame(cam, gaussian_scaling=scaling, sh_degree=0)
+    ref = orc.view_render(P, cam, scaling, 0, 1)
+    assert np.array_equal(img, ref["rgba"].reshape(img.shape))
