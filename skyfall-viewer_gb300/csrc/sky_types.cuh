@@ -116,6 +116,7 @@ struct DevBuffers {
   float* importance;      // 4 per Gaussian: sum, count, max radius, 0
   const StepParams* sp;
   DevStatus* status;
+  float neg_zero = -0.0f;  // for mul2_rounded
 };
 
 }  // namespace sky
