@@ -153,7 +153,7 @@ struct Context {
   Buf offsets, loss_partials, color, alpha, tfinal, last, residual, targets, sort_mem;
   Buf flags, flag_scan, d_sp, d_st;
   // densification statistics (float4 per Gaussian) and multi-view scores
-  Buf imp_stats, dens_accum, score_imp, score_prune, score_counts, metric_l1, metric_part,
+  Buf imp_stats, dens_accum, score_imp, score_prune, score_counts, metric_part,
       metric_stats, item_sums;
   bool scores_valid = false;  // scores belong to (scores_iter, current scene)
   uint64_t scores_iter = 0;
@@ -752,8 +752,9 @@ std::vector<uint32_t> sample_cameras(Context* c) {
   return idx;
 }
 
-// generateMultiViewScores (:2758-2788): render the views in batches, then
-// per view in order: L1 map, its statistics, error-pixel hits per Gaussian.
+// generateMultiViewScores (:2758-2788): render the views in batches, then for
+// all views of a batch at once the statistics of their L1 values and the
+// error-pixel hits per (view, Gaussian), which are combined view by view.
 int score_views(Context* c, const std::vector<uint32_t>& views) {
   const uint32_t n = c->n;
   for (uint32_t v : views) {
@@ -763,39 +764,36 @@ int score_views(Context* c, const std::vector<uint32_t>& views) {
   cudaStream_t s = c->stream;
   TRY(dev_alloc(c, c->score_imp, (size_t)n * 4));
   TRY(dev_alloc(c, c->score_prune, (size_t)n * 4));
-  TRY(dev_alloc(c, c->score_counts, (size_t)n * 4));
+  // hits per (view, Gaussian) of one batch of views
+  const size_t max_batch = std::min<size_t>(kMaxViews, views.size());
+  TRY(dev_alloc(c, c->score_counts, max_batch * n * 4));
   TRY(dev_alloc(c, c->metric_stats, (size_t)kMaxViews * sizeof(MetricStats)));
   CK(cudaMemsetAsync(c->score_imp.p, 0, (size_t)n * 4, s));
   CK(cudaMemsetAsync(c->score_prune.p, 0, (size_t)n * 4, s));
-  CK(cudaMemsetAsync(c->score_counts.p, 0, (size_t)n * 4, s));
   MetricStats* st = (MetricStats*)c->metric_stats.p;
   for (size_t first = 0; first < views.size(); first += kMaxViews) {
     const uint32_t nb = (uint32_t)std::min<size_t>(kMaxViews, views.size() - first);
     TRY(run_views(c, views.data() + first, nb, kRender, nullptr));
     DevBuffers b = make_buffers(c);
-    for (uint32_t v = 0; v < nb; ++v) {
-      const ViewInfo& vi = c->h_sp->views[v];
-      const uint32_t npx = vi.width * vi.height;
-      const uint32_t blocks = stat_blocks(npx);
-      TRY(dev_alloc(c, c->metric_l1, (size_t)npx * 4));
-      // partials: blocks f32 minima, blocks f32 maxima, then blocks f64 sums
-      // at byte offset 8 * blocks of the (256-byte aligned) allocation, so the
-      // f64 array is 8-byte aligned for every block count
-      TRY(dev_alloc(c, c->metric_part, (size_t)blocks * 16));
-      float* pmin = (float*)c->metric_part.p;
-      float* pmax = pmin + blocks;
-      double* psum = (double*)(pmax + blocks);
-      if ((reinterpret_cast<uintptr_t>(psum) & 7u) != 0u)
-        return fail(SKY_ERR_STATE, "metric partials misaligned");
-      launch_metric_map(b.color, b.targets, vi.pixel_base, vi.target_base, npx,
-                        (float*)c->metric_l1.p, s);
-      launch_metric_stats((const float*)c->metric_l1.p, npx, pmin, pmax, psum, blocks, st + v, s);
-      launch_metric_accum(b, v, npx, (const float*)c->metric_l1.p, st + v, 0.1f,
-                          (uint32_t*)c->score_counts.p, s);
-      launch_metric_combine((uint32_t*)c->score_counts.p, n, st + v, (uint32_t*)c->score_imp.p,
-                            (float*)c->score_prune.p, s);
-      c->launches += 5;
-    }
+    uint32_t max_px = 0;
+    for (uint32_t v = 0; v < nb; ++v)
+      max_px = std::max(max_px, c->h_sp->views[v].width * c->h_sp->views[v].height);
+    const uint32_t blocks = stat_blocks(max_px), slots = blocks * nb;
+    // partials: per view `blocks` f32 minima, then the f32 maxima, then the
+    // f64 sums at byte offset 8 * slots of the (256-byte aligned) allocation,
+    // so the f64 array is 8-byte aligned for every block count
+    TRY(dev_alloc(c, c->metric_part, (size_t)slots * 16));
+    float* pmin = (float*)c->metric_part.p;
+    float* pmax = pmin + slots;
+    double* psum = (double*)(pmax + slots);
+    if ((reinterpret_cast<uintptr_t>(psum) & 7u) != 0u)
+      return fail(SKY_ERR_STATE, "metric partials misaligned");
+    CK(cudaMemsetAsync(c->score_counts.p, 0, (size_t)nb * n * 4, s));
+    launch_metric_stats(b, nb, pmin, pmax, psum, blocks, st, s);
+    launch_metric_accum(b, c->last_tiles, c->cfg.tile_size, st, 0.1f, (uint32_t*)c->score_counts.p, s);
+    launch_metric_combine((const uint32_t*)c->score_counts.p, n, nb, st, (uint32_t*)c->score_imp.p,
+                          (float*)c->score_prune.p, s);
+    c->launches += 4;
   }
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(s));
@@ -1177,7 +1175,7 @@ int sky_destroy(void* p) {
                 &c->tile_grads, &c->gsum54, &c->offsets, &c->loss_partials, &c->color,
                 &c->alpha, &c->tfinal, &c->last, &c->residual, &c->targets, &c->sort_mem, &c->flags,
                 &c->flag_scan, &c->d_sp, &c->d_st, &c->imp_stats, &c->dens_accum,
-                &c->score_imp, &c->score_prune, &c->score_counts, &c->metric_l1,
+                &c->score_imp, &c->score_prune, &c->score_counts,
                 &c->metric_part, &c->metric_stats, &c->v_splats, &c->v_keys, &c->v_counts,
                 &c->v_rects, &c->v_order, &c->v_ksorted, &c->v_cum, &c->v_csorted, &c->v_bsums,
                 &c->v_misc, &c->v_tkeys, &c->v_gidx, &c->v_tkeys_s, &c->v_gidx_s, &c->v_offsets,

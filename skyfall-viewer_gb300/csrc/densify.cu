@@ -17,30 +17,21 @@ namespace {
 
 constexpr uint32_t kFull = 0xFFFFFFFFu;
 
-// Per-pixel L1 map of one view (compute_metric_map, metric-map.wgsl:32-50).
-// The target is sampled at texel centres of an image of the view's size, so
-// the bilinear sample is the texel itself.
-__global__ void k_metric_map(const float4* __restrict__ color, const float4* __restrict__ target,
-                             uint32_t pixel_base, uint32_t target_base, uint32_t npx,
-                             float* __restrict__ l1) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= npx) return;
-  const float4 p = color[(size_t)pixel_base + i];
-  const float4 t = target[(size_t)target_base + i];
-  const float dr = fabsf(p.x - t.x), dg = fabsf(p.y - t.y), db = fabsf(p.z - t.z);
-  l1[i] = ((dr + dg) + db) / 3.0f;
-}
-
-// Block partials of min, max (order-independent) and the f64 sum of the map.
+// Block partials of the min, max (order-independent) and f64 sum of a view's
+// L1 values (metric_l1), one row of blocks per view.  The values are formed
+// from the images here and again by k_metric_accum: storing them between the
+// two would cost the traffic of reading one of the images again.
 __global__ void __launch_bounds__(256)
-k_metric_partials(const float* __restrict__ l1, uint32_t npx, float* __restrict__ pmin,
-                  float* __restrict__ pmax, double* __restrict__ psum) {
+k_metric_partials(DevBuffers b, float* __restrict__ pmin, float* __restrict__ pmax,
+                  double* __restrict__ psum) {
   __shared__ float smin[8], smax[8];
   __shared__ double ssum[8];
+  const ViewInfo& vi = b.sp->views[blockIdx.y];
+  const uint32_t npx = vi.width * vi.height;
   float mn = INFINITY, mx = -INFINITY;
   double sm = 0.0;
   for (uint32_t i = blockIdx.x * 256 + threadIdx.x; i < npx; i += gridDim.x * 256) {
-    const float v = l1[i];
+    const float v = metric_l1(b.color[(size_t)vi.pixel_base + i], b.targets[(size_t)vi.target_base + i]);
     if (!isfinite(v)) continue;  // computePixelLossStats skips non-finite values
     mn = fminf(mn, v);
     mx = fmaxf(mx, v);
@@ -60,30 +51,43 @@ k_metric_partials(const float* __restrict__ l1, uint32_t npx, float* __restrict_
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    float a = smin[0], b = smax[0];
+    float a = smin[0], c = smax[0];
     double t = ssum[0];
     for (int k = 1; k < 8; ++k) {
       a = fminf(a, smin[k]);
-      b = fmaxf(b, smax[k]);
+      c = fmaxf(c, smax[k]);
       t += ssum[k];
     }
-    pmin[blockIdx.x] = a;
-    pmax[blockIdx.x] = b;
-    psum[blockIdx.x] = t;
+    const uint32_t slot = blockIdx.y * gridDim.x + blockIdx.x;
+    pmin[slot] = a;
+    pmax[slot] = c;
+    psum[slot] = t;
   }
 }
 
-__global__ void k_metric_final(const float* __restrict__ pmin, const float* __restrict__ pmax,
-                               const double* __restrict__ psum, uint32_t nblocks, uint32_t npx,
-                               MetricStats* __restrict__ out) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
+// One warp per view adds its partials, 32 chains at a time (one thread
+// walking 600 partials waited on each f64 addition: 51 us a view).
+__global__ void __launch_bounds__(32)
+k_metric_final(DevBuffers b, const float* __restrict__ pmin, const float* __restrict__ pmax,
+               const double* __restrict__ psum, uint32_t nblocks, MetricStats* __restrict__ stats) {
+  const ViewInfo& vi = b.sp->views[blockIdx.x];
+  const uint32_t npx = vi.width * vi.height;
+  const size_t base = (size_t)blockIdx.x * nblocks;
   float mn = INFINITY, mx = -INFINITY;
   double sm = 0.0;
-  for (uint32_t k = 0; k < nblocks; ++k) {
-    mn = fminf(mn, pmin[k]);
-    mx = fmaxf(mx, pmax[k]);
-    sm += psum[k];
+  for (uint32_t k = threadIdx.x; k < nblocks; k += 32) {
+    mn = fminf(mn, pmin[base + k]);
+    mx = fmaxf(mx, pmax[base + k]);
+    sm += psum[base + k];
   }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    mn = fminf(mn, __shfl_xor_sync(kFull, mn, o));
+    mx = fmaxf(mx, __shfl_xor_sync(kFull, mx, o));
+    sm += __shfl_xor_sync(kFull, sm, o);
+  }
+  if (threadIdx.x != 0) return;
+  MetricStats* out = stats + blockIdx.x;
   out->min_value = mn;
   out->max_value = mx;
   out->pad = 0.0f;
@@ -92,48 +96,22 @@ __global__ void k_metric_final(const float* __restrict__ pmin, const float* __re
   out->inv_range = mx > mn ? (float)(1.0 / ((double)mx - (double)mn)) : 0.0f;
 }
 
-// threshold_metric_map (:56-66) and accumulate_metric_counts (:86-147): for
-// every flagged pixel, each intersection of its tile up to the pixel's last
-// visited one whose Gaussian has 0 <= s <= 6 there adds one to that Gaussian.
-__global__ void __launch_bounds__(256)
-k_metric_accum(DevBuffers b, uint32_t view, const float* __restrict__ l1,
-               const MetricStats* __restrict__ st, float threshold, uint32_t* __restrict__ counts) {
-  const StepParams& sp = *b.sp;
-  const ViewInfo& vi = sp.views[view];
-  const uint32_t npx = vi.width * vi.height;
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= npx) return;
-  const float value = (l1[i] - st->min_value) * st->inv_range;
-  if (!(value > threshold)) return;
-  const uint32_t x = i % vi.width, y = i / vi.width;
-  const uint32_t ts = sp.tile_size;
-  const uint32_t tile = vi.tile_base + (y / ts) * vi.tiles_x + (x / ts);
-  const uint32_t start = b.offsets[tile], end = b.offsets[tile + 1];
-  if (start >= end) return;
-  const uint32_t last = b.last[(size_t)vi.pixel_base + i];
-  if (last < start) return;
-  const uint32_t fin = min(last, end - 1);
-  const float px = (float)x + 0.5f, py = (float)y + 0.5f;
-  for (uint32_t k = start; k <= fin; ++k) {
-    const uint32_t r = b.flatten[k];
-    const float4 q0 = b.records[(size_t)r * 3 + 0];
-    const float cc = b.records[(size_t)r * 3 + 1].x;
-    const float dx = px - q0.x, dy = py - q0.y;
-    const float s = 0.5f * ((q0.z * dx) * dx + (cc * dy) * dy) + (q0.w * dx) * dy;
-    if (s < 0.0f || s > 6.0f) continue;
-    atomicAdd(&counts[r % sp.n], 1u);
-  }
-}
-
-__global__ void k_metric_combine(uint32_t* __restrict__ counts, uint32_t n,
+// counts: per (view, Gaussian) item; the views are added in order.
+__global__ void k_metric_combine(const uint32_t* __restrict__ counts, uint32_t n, uint32_t views,
                                  const MetricStats* __restrict__ st,
                                  uint32_t* __restrict__ importance, float* __restrict__ pruning) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const uint32_t c = counts[i];
-  importance[i] += c;
-  pruning[i] = (float)((double)pruning[i] + (double)c * st->mean);
-  counts[i] = 0u;
+  uint32_t imp = importance[i];
+  float pr = pruning[i];
+  for (uint32_t v = 0; v < views; ++v) {
+    const uint32_t c = counts[(size_t)v * n + i];
+    if (c == 0u) continue;  // (the means are finite)
+    imp += c;
+    pr = (float)((double)pr + (double)c * st[v].mean);
+  }
+  importance[i] = imp;
+  pruning[i] = pr;
 }
 
 __device__ double max_sigma(const float* __restrict__ P, uint32_t stride, uint32_t i) {
@@ -380,26 +358,15 @@ uint32_t blocks_for(uint32_t n, uint32_t threads) { return (n + threads - 1) / t
 
 }  // namespace
 
-void launch_metric_map(const float4* color, const float4* target, uint32_t pixel_base,
-                       uint32_t target_base, uint32_t npx, float* l1, cudaStream_t s) {
-  if (npx)
-    k_metric_map<<<blocks_for(npx, 256), 256, 0, s>>>(color, target, pixel_base, target_base, npx, l1);
-}
-
-void launch_metric_stats(const float* l1, uint32_t npx, float* pmin, float* pmax, double* psum,
+void launch_metric_stats(const DevBuffers& b, uint32_t views, float* pmin, float* pmax, double* psum,
                          uint32_t nblocks, MetricStats* out, cudaStream_t s) {
-  k_metric_partials<<<nblocks, 256, 0, s>>>(l1, npx, pmin, pmax, psum);
-  k_metric_final<<<1, 32, 0, s>>>(pmin, pmax, psum, nblocks, npx, out);
+  k_metric_partials<<<dim3(nblocks, views), 256, 0, s>>>(b, pmin, pmax, psum);
+  k_metric_final<<<views, 32, 0, s>>>(b, pmin, pmax, psum, nblocks, out);
 }
 
-void launch_metric_accum(const DevBuffers& b, uint32_t view, uint32_t npx, const float* l1,
-                         const MetricStats* st, float threshold, uint32_t* counts, cudaStream_t s) {
-  if (npx) k_metric_accum<<<blocks_for(npx, 256), 256, 0, s>>>(b, view, l1, st, threshold, counts);
-}
-
-void launch_metric_combine(uint32_t* counts, uint32_t n, const MetricStats* st,
+void launch_metric_combine(const uint32_t* counts, uint32_t n, uint32_t views, const MetricStats* st,
                            uint32_t* importance, float* pruning, cudaStream_t s) {
-  if (n) k_metric_combine<<<blocks_for(n, 256), 256, 0, s>>>(counts, n, st, importance, pruning);
+  if (n) k_metric_combine<<<blocks_for(n, 256), 256, 0, s>>>(counts, n, views, st, importance, pruning);
 }
 
 void launch_densify_decide(const float* P, uint32_t stride, uint32_t n, const float4* accum,

@@ -45,16 +45,25 @@ __host__ __device__ inline double counter_uniform(uint64_t seed, uint64_t iterat
   return ((double)(z >> 11) + 0.5) * (1.0 / 9007199254740992.0);
 }
 
-void launch_metric_map(const float4* color, const float4* target, uint32_t pixel_base,
-                       uint32_t target_base, uint32_t npx, float* l1, cudaStream_t s);
-// nblocks partial slots in pmin/pmax/psum; result in *out.
-void launch_metric_stats(const float* l1, uint32_t npx, float* pmin, float* pmax, double* psum,
+// Per-pixel L1 value of a view (compute_metric_map, metric-map.wgsl:32-50).
+// The target is sampled at texel centres of an image of the view's size, so
+// the bilinear sample is the texel itself.
+__device__ __forceinline__ float metric_l1(const float4& p, const float4& t) {
+  const float dr = fabsf(p.x - t.x), dg = fabsf(p.y - t.y), db = fabsf(p.z - t.z);
+  return ((dr + dg) + db) / 3.0f;
+}
+
+// The views of the last pass: statistics of their L1 values (nblocks partial
+// slots per view in pmin/pmax/psum), out[v] per view.
+void launch_metric_stats(const DevBuffers& b, uint32_t views, float* pmin, float* pmax, double* psum,
                          uint32_t nblocks, MetricStats* out, cudaStream_t s);
-void launch_metric_accum(const DevBuffers& b, uint32_t view, uint32_t npx, const float* l1,
+// (kernels.cu) counts[item] += the flagged pixels each (view, Gaussian) item
+// reaches; counts holds views * n words.
+void launch_metric_accum(const DevBuffers& b, uint32_t tiles, uint32_t tile_size,
                          const MetricStats* st, float threshold, uint32_t* counts, cudaStream_t s);
-// importance += counts, pruning += counts * mean (f32, as the reference's
-// Float32Array), counts reset to 0.
-void launch_metric_combine(uint32_t* counts, uint32_t n, const MetricStats* st,
+// Per view in order: importance += counts, pruning += counts * mean (f32, as
+// the reference's Float32Array).
+void launch_metric_combine(const uint32_t* counts, uint32_t n, uint32_t views, const MetricStats* st,
                            uint32_t* importance, float* pruning, cudaStream_t s);
 
 // action (0 none, 1 clone, 2 split) and a 64-bit sort key (two u32 halves)

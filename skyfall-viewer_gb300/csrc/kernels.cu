@@ -2,6 +2,7 @@
 // tile ranges, the tiled forward rasterizer with the fused loss, the tiled
 // backward (exact and reference modes), and the fused geometry adjoint +
 // Adam.  Sort lives in sort.cu.  See kernels.cuh for the launch interface.
+#include "densify.cuh"
 #include "kernels.cuh"
 #include "project.cuh"
 
@@ -11,6 +12,7 @@ namespace sky {
 namespace {
 
 constexpr uint32_t kFull = 0xFFFFFFFFu;
+constexpr float kMetricS = 6.0f;  // multi-view scores: s of a Gaussian's reach
 
 SKY_DEV float load_plane(const float* __restrict__ P, uint32_t stride, int plane, uint32_t g,
                          bool r16) {
@@ -654,10 +656,8 @@ SKY_DEV uint32_t block_mask(float4 r0, float4 r2, uint32_t x0, uint32_t y0) {
 // so the block's warp would do nothing with the splat.  Worse-conditioned
 // conics keep the bounding-box mask.
 template <int TS, int BW, int BH>
-SKY_DEV uint32_t ellipse_block_mask(float4 r0, float4 r1, float4 r2, uint32_t x0, uint32_t y0) {
+SKY_DEV uint32_t ellipse_strips(const EllipseRows& e, uint32_t x0, uint32_t y0) {
   constexpr int NCOL = TS / BW, NROW = TS / BH;
-  EllipseRows e;  // x and y exchanged: e.mx is the mean's y, e.my its x
-  if (!ellipse_rows(r0.y, r0.x, r1.x, r0.w, r0.z, r2.y, e)) return block_mask<TS, BW, BH>(r0, r2, x0, y0);
   uint32_t keep = 0u;
 #pragma unroll
   for (int bc = 0; bc < NCOL; ++bc) {
@@ -672,6 +672,23 @@ SKY_DEV uint32_t ellipse_block_mask(float4 r0, float4 r1, float4 r2, uint32_t x0
     }
   }
   return keep;
+}
+
+template <int TS, int BW, int BH>
+SKY_DEV uint32_t ellipse_block_mask(float4 r0, float4 r1, float4 r2, uint32_t x0, uint32_t y0) {
+  EllipseRows e;
+  if (!ellipse_rows(r0.y, r0.x, r1.x, r0.w, r0.z, r2.y, e)) return block_mask<TS, BW, BH>(r0, r2, x0, y0);
+  return ellipse_strips<TS, BW, BH>(e, x0, y0);
+}
+
+// The blocks of the ellipse s <= kMetricS (every block where the conic is
+// worse conditioned or not finite).
+template <int TS, int BW, int BH>
+SKY_DEV uint32_t metric_mask(float4 q0, float cc, uint32_t x0, uint32_t y0) {
+  constexpr uint32_t kAll = TS / BW * (TS / BH) >= 32 ? kFull : (1u << (TS / BW * (TS / BH))) - 1u;
+  EllipseRows e;
+  if (!(q0.z + cc < 1e30f) || !ellipse_rows(q0.y, q0.x, cc, q0.w, q0.z, kMetricS, e)) return kAll;
+  return ellipse_strips<TS, BW, BH>(e, x0, y0);
 }
 
 template <int TS, int RPW = 32 / TS>
@@ -1797,6 +1814,94 @@ __global__ void __launch_bounds__(TS* TS) k_backward_ref(DevBuffers b) {
 }
 
 // ---------------------------------------------------------------------------
+// Multi-view scores: threshold_metric_map and accumulate_metric_counts
+// (metric-map.wgsl:56-66, :86-147).  For every flagged pixel, each
+// intersection of its tile up to the pixel's last visited one whose Gaussian
+// has 0 <= s <= 6 there adds one to that item.  One CTA per tile of the step,
+// as the forward: staged records, block masks (of the ellipse s <= 6) and
+// per-warp lists; a warp's pixels are counted by ballot, the tile's warps add
+// in shared memory, and each staged splat costs at most one global atomic.
+// 10 views of 500k Gaussians at 720p: 5441 -> 1059 us against one thread per
+// pixel walking the list in global memory with an atomic per hit.
+// ---------------------------------------------------------------------------
+template <int TS>
+__global__ void __launch_bounds__(TS* TS)
+k_metric_accum(DevBuffers b, const MetricStats* __restrict__ stats, float threshold,
+               uint32_t* __restrict__ counts) {
+  constexpr int NT = TS * TS, NW = NT / 32, FB = NT < 256 ? NT : 256;
+  __shared__ float4 s_rec[FB];   // mean, conic a, b
+  __shared__ float s_c[FB];      // conic c
+  __shared__ uint32_t s_mask[FB], s_cnt[FB];
+  __shared__ uint8_t s_list[NW][FB];
+  __shared__ int s_fin[NW];
+  const StepParams& sp = *b.sp;
+  const uint32_t tile = blockIdx.x;
+  if (tile >= sp.num_tiles || capacity_failed(b.status)) return;
+  const uint32_t start = b.offsets[tile], end = b.offsets[tile + 1];
+  if (start >= end) return;
+  const int v = find_view(sp, tile);
+  const ViewInfo& vi = sp.views[v];
+  const uint32_t local = tile - vi.tile_base;
+  const uint32_t tx = local % vi.tiles_x, ty = local / vi.tiles_x;
+  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t x = tx * TS + 8u * (warp % (TS / 8)) + (lane & 7u);
+  const uint32_t y = ty * TS + 4u * (warp / (TS / 8)) + (lane >> 3);
+  const float px = (float)x + 0.5f, py = (float)y + 0.5f;
+  int fin = -1;  // the pixel's last intersection, -1: not flagged
+  if (x < vi.width && y < vi.height) {
+    const uint32_t i = y * vi.width + x;
+    const size_t p = (size_t)vi.pixel_base + i;
+    const float l1 = metric_l1(b.color[p], b.targets[(size_t)vi.target_base + i]);
+    const float value = (l1 - stats[v].min_value) * stats[v].inv_range;
+    const uint32_t last = b.last[p];
+    if (value > threshold && last >= start) fin = (int)min(last, end - 1);
+  }
+  int wfin = fin;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) wfin = max(wfin, __shfl_xor_sync(kFull, wfin, o));
+  if (lane == 0) s_fin[warp] = wfin;
+  __syncthreads();
+  int tfin = s_fin[0];
+  for (int w = 1; w < NW; ++w) tfin = max(tfin, s_fin[w]);
+  const uint32_t wbit = 1u << warp, lt = (1u << lane) - 1u;
+  for (int bs = (int)start; bs <= tfin; bs += FB) {
+    const int cnt = min(FB, tfin - bs + 1);
+    __syncthreads();
+    uint32_t item = 0;  // of the splat this thread stages and later counts (FB <= NT)
+    if ((int)tid < cnt) {
+      item = b.flatten[bs + (int)tid];
+      const float4 q0 = b.records[(size_t)item * 3 + 0];
+      const float cc = b.records[(size_t)item * 3 + 1].x;
+      s_rec[tid] = q0;
+      s_c[tid] = cc;
+      s_cnt[tid] = 0u;
+      s_mask[tid] = metric_mask<TS, 8, 4>(q0, cc, tx * TS, ty * TS);
+    }
+    __syncthreads();
+    uint32_t nlist = 0;
+    for (int base = 0; base < cnt; base += 32) {
+      const int j = base + (int)lane;
+      const bool in = j < cnt && (s_mask[j] & wbit) && bs + j <= wfin;
+      const uint32_t m = __ballot_sync(kFull, in);
+      if (in) s_list[warp][nlist + __popc(m & lt)] = (uint8_t)j;
+      nlist += __popc(m);
+    }
+    __syncwarp();
+    for (uint32_t li = 0; li < nlist; ++li) {
+      const int j = s_list[warp][li];
+      const float4 q0 = s_rec[j];
+      const float dx = px - q0.x, dy = py - q0.y;
+      const float s = 0.5f * ((q0.z * dx) * dx + (s_c[j] * dy) * dy) + (q0.w * dx) * dy;
+      const bool hit = bs + j <= fin && !(s < 0.0f || s > kMetricS);
+      const uint32_t hits = __popc(__ballot_sync(kFull, hit));
+      if (lane == 0 && hits) atomicAdd(&s_cnt[j], hits);
+    }
+    __syncthreads();
+    if ((int)tid < cnt && s_cnt[tid]) atomicAdd(&counts[item], s_cnt[tid]);
+  }
+}
+
+// ---------------------------------------------------------------------------
 // Geometry adjoint + SH chain + Adam, one thread per Gaussian.  For each view
 // of the step: sum the Gaussian's per-intersection partials (contiguous in
 // emission order, summed in order), then back-propagate dL/d(colour, logit,
@@ -2408,6 +2513,16 @@ void launch_backward(const DevBuffers& b, uint32_t max_tiles, uint32_t ts, uint3
       case 32: k_backward_ref<32><<<max_tiles, 1024, 0, s>>>(b); break;
       default: k_backward_ref<16><<<max_tiles, 256, 0, s>>>(b); break;
     }
+  }
+}
+
+void launch_metric_accum(const DevBuffers& b, uint32_t tiles, uint32_t ts, const MetricStats* st,
+                         float threshold, uint32_t* counts, cudaStream_t s) {
+  if (tiles == 0) return;
+  switch (ts) {
+    case 8: k_metric_accum<8><<<tiles, 64, 0, s>>>(b, st, threshold, counts); break;
+    case 32: k_metric_accum<32><<<tiles, 1024, 0, s>>>(b, st, threshold, counts); break;
+    default: k_metric_accum<16><<<tiles, 256, 0, s>>>(b, st, threshold, counts); break;
   }
 }
 
