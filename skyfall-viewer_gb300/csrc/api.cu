@@ -154,7 +154,7 @@ struct Context {
   Buf flags, flag_scan, d_sp, d_st;
   // densification statistics (float4 per Gaussian) and multi-view scores
   Buf imp_stats, dens_accum, score_imp, score_prune, score_counts, metric_part,
-      metric_stats, item_sums;
+      metric_stats, item_sums, sh_items;
   bool scores_valid = false;  // scores belong to (scores_iter, current scene)
   uint64_t scores_iter = 0;
   uint32_t scores_n = 0, scores_views = 0;
@@ -273,6 +273,7 @@ DevBuffers make_buffers(Context* c) {
   b.reached = (uint8_t*)c->reached.p;
   b.partials = (float4*)c->partials.p;
   b.item_sums = (float4*)c->item_sums.p;
+  b.sh_items = (float*)c->sh_items.p;
   b.tile_grads = (int32_t*)c->tile_grads.p;
   b.gsum54 = (long long*)c->gsum54.p;
   b.offsets = (uint32_t*)c->offsets.p;
@@ -422,8 +423,7 @@ int enqueue(Context* c, const Shape& sh, bool sizing_sync, uint64_t& launches, u
       launch_item_sums(b, items, s);
       ++launches;
     }
-    launch_geom_adam(b, sh.n, s);
-    launches += 2;
+    launches += 1 + launch_geom_adam(b, sh.n, sh.nv, sh.mode == kTrain && !sh.ref, s);
   } else {
     TRY(mark(7));
   }
@@ -540,6 +540,8 @@ int run_views(Context* c, const uint32_t* cams, uint32_t nv, Mode mode, SkyStepS
   const bool ref = cfg.backward_mode == SKY_BWD_REFERENCE;
   if (ref && mode >= kBackward) TRY(dev_alloc(c, c->gsum54, items * 54 * 8));
   if (!ref && mode >= kBackward) TRY(dev_alloc(c, c->item_sums, items * 48));
+  if (!ref && mode == kTrain && nv <= (uint32_t)kFewViews)
+    TRY(dev_alloc(c, c->sh_items, (size_t)nv * 6 * c->stride * 4));
   if (c->icap == 0) TRY(ensure_isect(c, 1u << 16));
   // schedules
   uint64_t it = c->iteration + (mode == kTrain ? 1 : 0);
@@ -1179,7 +1181,7 @@ int sky_destroy(void* p) {
                 &c->metric_part, &c->metric_stats, &c->v_splats, &c->v_keys, &c->v_counts,
                 &c->v_rects, &c->v_order, &c->v_ksorted, &c->v_cum, &c->v_csorted, &c->v_bsums,
                 &c->v_misc, &c->v_tkeys, &c->v_gidx, &c->v_tkeys_s, &c->v_gidx_s, &c->v_offsets,
-                &c->v_rgba, &c->v_sort, &c->item_sums};
+                &c->v_rgba, &c->v_sort, &c->item_sums, &c->sh_items};
   for (Buf* b : all) dev_free(c, *b);
   drop_graph(c);
   for (int k = 0; k <= SKY_NUM_STAGES; ++k)

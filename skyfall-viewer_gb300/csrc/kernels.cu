@@ -2091,9 +2091,16 @@ SKY_DEV void adam_vals(float& p, float& m1, float& m2, float g, float lr, const 
   const float c = k.b2 * m2;
   const float d = (k.omb2 * g) * g;
   const float nm2 = c + d;
-  const float denom = sqrtf(nm2) * k.bc2_sqrt_rcp + k.eps;
+  // 0 takes the slow paths of the IEEE square root and quotient, and a
+  // Gaussian no pixel has reached yet has only zeros: both get 1 instead, and
+  // the known result (0 / denom keeps its sign for denom > 0).
+  const bool z2 = nm2 == 0.0f;
+  const float root = sqrtf(z2 ? 1.0f : nm2);
+  const float denom = (z2 ? 0.0f : root) * k.bc2_sqrt_rcp + k.eps;
   const float step = lr * k.bc1_rcp;
-  p = p - step * (nm1 / denom);
+  const bool z1 = nm1 == 0.0f && denom > 0.0f;
+  const float q = (z1 ? 1.0f : nm1) / denom;
+  p = p - step * (z1 ? nm1 : q);
   m1 = nm1;
   m2 = nm2;
 }
@@ -2182,30 +2189,41 @@ __global__ void __launch_bounds__(256) k_item_sums(DevBuffers b) {
   }
 }
 
-// Dynamic shared memory of k_geom_adam: SH values and SH-gradient
+// Dynamic shared memory of k_geom_adam: SH values and, unless FEW, SH-gradient
 // accumulators (48 x threads f32 each), two buffers of the threads' item
 // sums (3 float4 per thread) and two of their (depth, radius) pairs.
-constexpr size_t kGeomSmem =
-    (size_t)96 * kGeomThreads * 4 + (size_t)2 * 3 * kGeomThreads * 16 + (size_t)2 * kGeomThreads * 8;
+template <bool FEW>
+constexpr size_t geom_smem() {
+  return (size_t)(FEW ? 48 : 96) * kGeomThreads * 4 + (size_t)2 * 3 * kGeomThreads * 16 +
+         (size_t)2 * kGeomThreads * 8;
+}
 
 // SH values and SH-gradient accumulators live in shared memory (one column
 // per thread, conflict-free), as do the item sums of the next view, copied
 // asynchronously while the current view's adjoint runs, and the step's
 // cameras; three blocks per multiprocessor resident (168 registers, 60 KB of
-// dynamic and 12 KB of static shared memory each).
+// dynamic and 12 KB of static shared memory each), four if FEW (128 registers;
+// three: 12 % slower).  Issue slots 52 %, DRAM 41 % busy: 3670 instructions per
+// Gaussian and view of arithmetic that keeps the reference's order.
+// FEW: exact-mode training steps of at most kFewViews views.  The SH
+// gradients are not accumulated: on SH-update steps each item's view
+// direction and unclamped colour gradient go to b.sh_items, and k_sh_adam
+// forms the gradients from them.
 static_assert(sizeof(ViewInfo) % 4 == 0, "cameras are copied as 32-bit words");
-__global__ void __launch_bounds__(kGeomThreads, 3) k_geom_adam(DevBuffers b) {
+template <bool FEW>
+__global__ void __launch_bounds__(kGeomThreads, FEW ? 4 : 3) k_geom_adam(DevBuffers b) {
   extern __shared__ float4 s_dyn[];
   float* const s_base = reinterpret_cast<float*>(s_dyn);
+  constexpr int kShRows = FEW ? 48 : 96;
   float (*s_sh)[kGeomThreads] = reinterpret_cast<float (*)[kGeomThreads]>(s_base);
-  float (*s_gsh)[kGeomThreads] = reinterpret_cast<float (*)[kGeomThreads]>(s_base + 48 * kGeomThreads);
+  float (*s_gsh)[kGeomThreads] = reinterpret_cast<float (*)[kGeomThreads]>(s_base + 48 * kGeomThreads);  // !FEW
   float4 (*s_is)[3][kGeomThreads] =
-      reinterpret_cast<float4 (*)[3][kGeomThreads]>(s_base + 96 * kGeomThreads);
+      reinterpret_cast<float4 (*)[3][kGeomThreads]>(s_base + kShRows * kGeomThreads);
   float2 (*s_aux)[kGeomThreads] =
-      reinterpret_cast<float2 (*)[kGeomThreads]>(s_base + 96 * kGeomThreads + 2 * 3 * kGeomThreads * 4);
+      reinterpret_cast<float2 (*)[kGeomThreads]>(s_base + kShRows * kGeomThreads + 2 * 3 * kGeomThreads * 4);
   const StepParams& sp = *b.sp;
   // the step's cameras, read by every thread in every view iteration
-  __shared__ ViewInfo s_views[kMaxViews];
+  __shared__ ViewInfo s_views[FEW ? kFewViews : kMaxViews];
   {
     const uint32_t words = sp.num_views * (uint32_t)(sizeof(ViewInfo) / 4);
     const uint32_t* src = reinterpret_cast<const uint32_t*>(sp.views);
@@ -2221,15 +2239,15 @@ __global__ void __launch_bounds__(kGeomThreads, 3) k_geom_adam(DevBuffers b) {
   const bool r16 = sp.round_f16 != 0;
   const int deg = (int)sp.sh_deg;
   const int ncoef = (deg + 1) * (deg + 1);
-  const bool ref = sp.bwd_mode != 0;
-  const bool need_sh_grads = sp.sh_update || sp.write_grads;
+  const bool ref = !FEW && sp.bwd_mode != 0;
+  const bool need_sh_grads = sp.sh_update || (!FEW && sp.write_grads);
   // the SH coefficients go to this thread's column of s_sh by asynchronous
   // copies, all in flight at once, then rounded in place
 #pragma unroll
   for (int k = 0; k < 48; ++k) {
     if (!ref && k < 3 * ncoef) cp_async4(&s_sh[k][t], &b.params[(size_t)(11 + k) * stride + g]);
     else s_sh[k][t] = 0.0f;
-    s_gsh[k][t] = 0.0f;
+    if constexpr (!FEW) s_gsh[k][t] = 0.0f;
   }
   cp_async_commit();
   float prm[11];
@@ -2310,6 +2328,13 @@ __global__ void __launch_bounds__(kGeomThreads, 3) k_geom_adam(DevBuffers b) {
         imp.z = fmax_(imp.z, s_aux[buf][t].y);
       }
     }
+    // the item's entry for k_sh_adam: colour gradient 0 until there is one
+    auto sh_item = [&](float x, float y, float z, float r, float gr_, float bl) {
+      const float e[6] = {x, y, z, r, gr_, bl};
+#pragma unroll
+      for (int k = 0; k < 6; ++k) b.sh_items[((size_t)v * 6 + k) * stride + g] = e[k];
+    };
+    if (FEW && need_sh_grads) sh_item(0.f, 0.f, 0.f, 0.f, 0.f, 0.f);
     if (cnt == 0) continue;
     float in9[9];
 #pragma unroll
@@ -2320,7 +2345,7 @@ __global__ void __launch_bounds__(kGeomThreads, 3) k_geom_adam(DevBuffers b) {
       in9[4] = a1.x; in9[5] = a1.y; in9[6] = a1.z; in9[7] = a1.w; in9[8] = a2.x;
 #pragma unroll
       for (int k = 0; k < 9; ++k) any = any || in9[k] != 0.0f;
-    } else {
+    } else if constexpr (!FEW) {
       const long long* sref = b.gsum54 + item * 54;
       const float sc = 1.0f / 65536.0f;
       in9[3] = (float)sref[0] * sc;
@@ -2355,7 +2380,12 @@ __global__ void __launch_bounds__(kGeomThreads, 3) k_geom_adam(DevBuffers b) {
     ProjOut o;
     view_color(get, pc, deg, !ref, o);
     geom_view(pc, o, vi, sp, gc.C3, in9, !ref, &s_sh[0][t], kGeomThreads, deg, gr, g3);
-    if (need_sh_grads && !ref) {
+    if constexpr (FEW) {
+      if (need_sh_grads) {
+        sh_item(o.dir[0], o.dir[1], o.dir[2], o.raw[0] > 0.0f ? in9[0] : 0.0f,
+                o.raw[1] > 0.0f ? in9[1] : 0.0f, o.raw[2] > 0.0f ? in9[2] : 0.0f);
+      }
+    } else if (need_sh_grads && !ref) {
       float Y[16];
       sh_basis(o.dir[0], o.dir[1], o.dir[2], deg, Y);
 #pragma unroll
@@ -2374,10 +2404,11 @@ __global__ void __launch_bounds__(kGeomThreads, 3) k_geom_adam(DevBuffers b) {
   geom_cov_final(prm, g3, gr);
   float g11[11] = {gr.pos[0], gr.pos[1], gr.pos[2], gr.ls[0], gr.ls[1], gr.ls[2],
                    gr.q[0],   gr.q[1],   gr.q[2],   gr.q[3],  gr.logit};
-  if (sp.write_grads) {
+  if (!FEW && sp.write_grads) {
 #pragma unroll
     for (int k = 0; k < 11; ++k) b.grads[(size_t)k * stride + g] = g11[k];
-    for (int k = 0; k < 48; ++k) b.grads[(size_t)(11 + k) * stride + g] = s_gsh[k][t];
+    if constexpr (!FEW)
+      for (int k = 0; k < 48; ++k) b.grads[(size_t)(11 + k) * stride + g] = s_gsh[k][t];
   }
   if (sp.apply_adam) {
     const AdamK ak = adam_consts(sp);
@@ -2388,7 +2419,7 @@ __global__ void __launch_bounds__(kGeomThreads, 3) k_geom_adam(DevBuffers b) {
                               g11[9], g11[10]}},
                     Vals<11>{{lr_pos, lr_pos, lr_pos, lr_scale, lr_scale, lr_scale, lr_rot, lr_rot,
                               lr_rot, lr_rot, lr_op}}, ak);
-    if (sp.sh_update) {
+    if constexpr (!FEW) if (sp.sh_update) {
 #pragma unroll
       for (int k0 = 0; k0 < 48; k0 += 12) {
         Vals<12> gv, lv;
@@ -2399,6 +2430,98 @@ __global__ void __launch_bounds__(kGeomThreads, 3) k_geom_adam(DevBuffers b) {
     }
   }
 }
+
+// Adam over the 48 SH planes after an exact step of few views.  A thread
+// takes four neighbouring Gaussians and kShCoefs coefficients (3 planes each):
+// it forms their SH gradients from the items' directions and colour gradients
+// (b.sh_items, k_geom_adam<true>), view by view, and updates the planes with
+// 16-byte accesses.  The blocks of one range of Gaussians follow one another,
+// so the items come from L2 but once.  Bound by memory: 1152 bytes per
+// Gaussian of parameters and moments at 5.6 TB/s (4M Gaussians, one view: 846
+// us; 1178 with 4-byte accesses, one Gaussian per thread).  The groups share
+// one copy of the update: unrolled into the eight cases its code missed the
+// instruction cache (1290 us).
+constexpr int kShAdamThreads = 128;
+constexpr int kShCoefs = 2;
+constexpr int kShGroups = 16 / kShCoefs;
+
+// Gradients of the coefficients [K0, K0 + kShCoefs) of Gaussians g .. g + 3
+// (those at or past n lie in the planes' padding: 0).
+template <int K0>
+SKY_DEV void sh_grads(const DevBuffers& b, const StepParams& sp, uint32_t g,
+                      float (&grad)[3 * kShCoefs][4]) {
+  const int deg = (int)sp.sh_deg;
+  const int ncoef = (deg + 1) * (deg + 1);
+#pragma unroll
+  for (int j = 0; j < 3 * kShCoefs; ++j)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) grad[j][q] = 0.0f;
+  if (K0 >= ncoef) return;
+  for (uint32_t v = 0; v < sp.num_views; ++v) {
+    float it[6][4];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+      const float4 x = *reinterpret_cast<const float4*>(&b.sh_items[((size_t)v * 6 + k) * sp.plane_stride + g]);
+      it[k][0] = x.x; it[k][1] = x.y; it[k][2] = x.z; it[k][3] = x.w;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      if (g + (uint32_t)q >= sp.n) continue;
+      float Y[16];  // (only the group's values are formed)
+      sh_basis(it[0][q], it[1][q], it[2][q], deg, Y);
+#pragma unroll
+      for (int k = 0; k < kShCoefs; ++k)
+        if (K0 + k < ncoef)
+#pragma unroll
+          for (int c = 0; c < 3; ++c) grad[3 * k + c][q] += Y[K0 + k] * it[3 + c][q];
+    }
+  }
+}
+
+__global__ void __launch_bounds__(kShAdamThreads, 4) k_sh_adam(DevBuffers b) {
+  const StepParams& sp = *b.sp;
+  if (!sp.sh_update || capacity_failed(b.status)) return;
+  const uint32_t work = (sp.n + 4 * kShAdamThreads - 1) / (4 * kShAdamThreads) * kShGroups;
+  for (uint32_t w = blockIdx.x; w < work; w += gridDim.x) {
+    const uint32_t g = 4u * (w / kShGroups * kShAdamThreads + threadIdx.x);
+    if (g >= sp.n) continue;
+    const int group = (int)(w % kShGroups);
+    float grad[3 * kShCoefs][4];
+    switch (group) {
+      case 0: sh_grads<0>(b, sp, g, grad); break;
+      case 1: sh_grads<1 * kShCoefs>(b, sp, g, grad); break;
+      case 2: sh_grads<2 * kShCoefs>(b, sp, g, grad); break;
+      case 3: sh_grads<3 * kShCoefs>(b, sp, g, grad); break;
+      case 4: sh_grads<4 * kShCoefs>(b, sp, g, grad); break;
+      case 5: sh_grads<5 * kShCoefs>(b, sp, g, grad); break;
+      case 6: sh_grads<6 * kShCoefs>(b, sp, g, grad); break;
+      default: sh_grads<7 * kShCoefs>(b, sp, g, grad); break;
+    }
+    const AdamK ak = adam_consts(sp);
+    const float lr = sp.lr_sh;
+    float4 P[3 * kShCoefs], M1[3 * kShCoefs], M2[3 * kShCoefs];
+    const size_t idx = (size_t)(11 + 3 * kShCoefs * group) * sp.plane_stride + g;
+#pragma unroll
+    for (int j = 0; j < 3 * kShCoefs; ++j) {
+      const size_t i = idx + (size_t)j * sp.plane_stride;
+      P[j] = *reinterpret_cast<const float4*>(&b.params[i]);
+      M1[j] = *reinterpret_cast<const float4*>(&b.m1[i]);
+      M2[j] = *reinterpret_cast<const float4*>(&b.m2[i]);
+    }
+#pragma unroll
+    for (int j = 0; j < 3 * kShCoefs; ++j) {
+      adam_vals(P[j].x, M1[j].x, M2[j].x, grad[j][0], lr, ak);
+      adam_vals(P[j].y, M1[j].y, M2[j].y, grad[j][1], lr, ak);
+      adam_vals(P[j].z, M1[j].z, M2[j].z, grad[j][2], lr, ak);
+      adam_vals(P[j].w, M1[j].w, M2[j].w, grad[j][3], lr, ak);
+      const size_t i = idx + (size_t)j * sp.plane_stride;
+      *reinterpret_cast<float4*>(&b.params[i]) = P[j];
+      *reinterpret_cast<float4*>(&b.m1[i]) = M1[j];
+      *reinterpret_cast<float4*>(&b.m2[i]) = M2[j];
+    }
+  }
+}
+static_assert(kShGroups == 8, "one case per group");
 
 }  // namespace
 
@@ -2526,18 +2649,34 @@ void launch_metric_accum(const DevBuffers& b, uint32_t tiles, uint32_t ts, const
   }
 }
 
-void launch_geom_adam(const DevBuffers& b, uint32_t n, cudaStream_t s) {
-  if (n == 0) return;
+template <bool FEW>
+void launch_geom_adam_as(const DevBuffers& b, uint32_t n, cudaStream_t s) {
   // per device: the opt-in above 48 KB of shared memory (idempotent, so two
   // threads that both see it unset both set it)
   static std::atomic<bool> smem_set[64];
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
   if (!smem_set[dev].load(std::memory_order_acquire)) {
-    cudaFuncSetAttribute(k_geom_adam, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGeomSmem);
+    cudaFuncSetAttribute(k_geom_adam<FEW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)geom_smem<FEW>());
     smem_set[dev].store(true, std::memory_order_release);
   }
-  k_geom_adam<<<(n + kGeomThreads - 1) / kGeomThreads, kGeomThreads, kGeomSmem, s>>>(b);
+  k_geom_adam<FEW><<<(n + kGeomThreads - 1) / kGeomThreads, kGeomThreads, geom_smem<FEW>(), s>>>(b);
+}
+
+int launch_geom_adam(const DevBuffers& b, uint32_t n, uint32_t views, bool train_exact, cudaStream_t s) {
+  if (n == 0) return 0;
+  if (!train_exact || views > (uint32_t)kFewViews) {
+    launch_geom_adam_as<false>(b, n, s);
+    return 1;
+  }
+  launch_geom_adam_as<true>(b, n, s);
+  // (a persistent grid: on the steps that leave the SH planes alone the launch
+  // is a few empty blocks)
+  const uint64_t work = (uint64_t)((n + 4 * kShAdamThreads - 1) / (4 * kShAdamThreads)) * kShGroups;
+  const uint32_t blocks = (uint32_t)std::min<uint64_t>(work, (uint64_t)sm_count() * 16);
+  k_sh_adam<<<blocks, kShAdamThreads, 0, s>>>(b);
+  return 2;
 }
 
 void launch_item_sums(const DevBuffers& b, uint64_t items, cudaStream_t s) {

@@ -27,7 +27,16 @@ void launch_forward(const DevBuffers& b, uint32_t max_tiles, uint32_t ts, uint32
 void launch_loss_final(const DevBuffers& b, cudaStream_t s);
 void launch_backward(const DevBuffers& b, uint32_t max_tiles, uint32_t ts, uint32_t bb, bool ref,
                      bool count, cudaStream_t s);
-void launch_geom_adam(const DevBuffers& b, uint32_t n, cudaStream_t s);
+// Training steps of at most kFewViews views in the exact backward mode hand the
+// SH part of Adam to a kernel of its own (b.sh_items, 24 bytes per item).  Both
+// parts then fit more warps, but that kernel reads every item once more: 1M
+// Gaussians, one kernel -> two: 1 view 542 -> 394 us, 4 views 688 -> 568, 6:
+// 788 -> 686, 16: 1323 -> 1213; 250k Gaussians: 16 views 340 -> 333, 32: 561 ->
+// 576, 64: 996 -> 1060.
+constexpr int kFewViews = 16;
+// train_exact: a training step (no gradients out) in the exact backward mode.
+// Returns the number of kernels launched.
+int launch_geom_adam(const DevBuffers& b, uint32_t n, uint32_t views, bool train_exact, cudaStream_t s);
 // Exact mode, before launch_geom_adam: per-item sums of the partials.
 void launch_item_sums(const DevBuffers& b, uint64_t items, cudaStream_t s);
 

@@ -102,6 +102,8 @@ struct DevBuffers {
   float4* partials;       // 3 float4 per intersection (emission order)
   uint8_t* reached;       // per emission index: 1 when the exact backward wrote its partial
   float4* item_sums;      // exact mode: 3 float4 per item, its partials summed
+  float* sh_items;        // steps of few views: per view 6 planes (stride plane_stride): view
+                          // direction and colour gradient of its items
   int32_t* tile_grads;    // reference mode: 54 per sorted intersection
   long long* gsum54;      // reference mode: 54 per item
   uint32_t* offsets;      // tile ranges, num_tiles + 1
