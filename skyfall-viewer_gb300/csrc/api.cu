@@ -1456,7 +1456,7 @@ int sky_knn_init(void* p, float scene_extent, float* density_out) {
   const uint32_t n = c->n;
   cudaStream_t s = c->stream;
   const float extent = scene_extent > 0.0f ? scene_extent : c->scene_extent;
-  TempBuf bounds(c), keys(c), ksorted(c), order(c), cstart(c), logs(c), dens(c), smem(c);
+  TempBuf bounds(c), keys(c), ksorted(c), order(c), cstart(c), logs(c), dens(c), smem(c), pos(c);
   TRY(dev_alloc(c, bounds.b, 64));
   uint32_t init[6];
   for (int k = 0; k < 6; ++k) init[k] = knn_bounds_init(k);
@@ -1501,6 +1501,7 @@ int sky_knn_init(void* p, float scene_extent, float* density_out) {
   TRY(dev_alloc(c, order.b, (size_t)n * 4));
   TRY(dev_alloc(c, cstart.b, ((size_t)g.cells + 1) * 4));
   TRY(dev_alloc(c, logs.b, (size_t)n * 4));
+  TRY(dev_alloc(c, pos.b, (size_t)n * 16));
   if (density_out) TRY(dev_alloc(c, dens.b, (size_t)n * 4));
   TRY(dev_alloc(c, smem.b, sort_scratch_bytes(n)));
   launch_knn_keys((const float*)c->params.p, c->stride, n, g, keys.as<uint32_t>(), s);
@@ -1511,10 +1512,10 @@ int sky_knn_init(void* p, float scene_extent, float* density_out) {
   CK(sort_pairs_launch(keys.as<uint32_t>(), nullptr, ksorted.as<uint32_t>(), order.as<uint32_t>(), seg,
                        n, std::max<uint32_t>(1, ceil_log2(g.cells)), sc, err, s));
   launch_knn_cell_ranges(ksorted.as<uint32_t>(), n, g.cells, cstart.as<uint32_t>(), s);
-  launch_knn_query((float*)c->params.p, c->stride, n, g, order.as<uint32_t>(), cstart.as<uint32_t>(),
-                   extent, dens.as<float>(), logs.as<float>(), s);
+  launch_knn_query((const float*)c->params.p, c->stride, n, g, order.as<uint32_t>(),
+                   cstart.as<uint32_t>(), pos.as<float4>(), extent, dens.as<float>(), logs.as<float>(), s);
   launch_knn_write((float*)c->params.p, c->stride, n, logs.as<float>(), s);
-  c->launches += 10;
+  c->launches += 11;
   CK(cudaGetLastError());
   uint32_t e = 0;
   CK(cudaMemcpyAsync(&e, err, 4, cudaMemcpyDeviceToHost, s));

@@ -28,9 +28,10 @@ void launch_knn_cell_ranges(const uint32_t* keys_sorted, uint32_t n, uint32_t ce
 // Three nearest other points of each point by an exact ring search over the
 // grid, then the reference's sigma rule; writes density (may be null) and
 // the f16 log sigma into the three scale planes of params (every other
-// plane is rounded through f16, as the reference's re-sync does).
-void launch_knn_query(float* params, uint32_t stride, uint32_t n, const KnnGrid& g,
-                      const uint32_t* order, const uint32_t* cell_start, float extent,
+// plane is rounded through f16, as the reference's re-sync does).  pos: n
+// float4 of scratch, the points in cell order.
+void launch_knn_query(const float* params, uint32_t stride, uint32_t n, const KnnGrid& g,
+                      const uint32_t* order, const uint32_t* cell_start, float4* pos, float extent,
                       float* density, float* log_sigma, cudaStream_t s);
 void launch_knn_write(float* params, uint32_t stride, uint32_t n, const float* log_sigma,
                       cudaStream_t s);
