@@ -126,18 +126,30 @@ k_sort_hist(const uint32_t* __restrict__ keys, SortSegment seg, int passes, int 
 }
 
 // Exclusive scan of each pass's 256 digit counts (one block per pass), and
-// trivial[pass] = 1 when one digit holds every key (the pass would be the
-// identity permutation, e.g. the high byte of the integer depth).
+// varying[pass]: the digit bits in which the keys differ.  0 when one digit
+// holds every key (the pass would be the identity permutation, e.g. the high
+// byte of the integer depth), and for passes below digit_lo.
 __global__ void __launch_bounds__(kRadix)
-k_sort_scan(uint32_t* __restrict__ hist, SortSegment seg, uint32_t* __restrict__ trivial,
-            int digit_lo) {
-  __shared__ uint32_t s_warp[kRadix / 32];
-  uint32_t begin, n;
-  seg_bounds(seg, begin, n);
+k_sort_scan(uint32_t* __restrict__ hist, uint32_t* __restrict__ varying, int digit_lo) {
+  __shared__ uint32_t s_warp[kRadix / 32], s_or[kRadix / 32], s_and[kRadix / 32];
   uint32_t* h = hist + blockIdx.x * kRadix;
   uint32_t v = h[threadIdx.x];
-  const int one_digit = __syncthreads_or(v == n);
-  if (threadIdx.x == 0) trivial[blockIdx.x] = (one_digit || (int)blockIdx.x < digit_lo) ? 1u : 0u;
+  const uint32_t any = __reduce_or_sync(0xFFFFFFFFu, v ? threadIdx.x : 0u);
+  const uint32_t all = __reduce_and_sync(0xFFFFFFFFu, v ? threadIdx.x : 0xFFu);
+  if ((threadIdx.x & 31) == 0) {
+    s_or[threadIdx.x >> 5] = any;
+    s_and[threadIdx.x >> 5] = all;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    uint32_t o = 0u, a = 0xFFu;
+    for (int w = 0; w < kRadix / 32; ++w) {
+      o |= s_or[w];
+      a &= s_and[w];
+    }
+    // (no key at all: o = 0, a = 0xFF)
+    varying[blockIdx.x] = (int)blockIdx.x < digit_lo ? 0u : (o & ~a);
+  }
   uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint32_t x = v;
 #pragma unroll
@@ -152,10 +164,15 @@ k_sort_scan(uint32_t* __restrict__ hist, SortSegment seg, uint32_t* __restrict__
   h[threadIdx.x] = x - v + add;
 }
 
-__global__ void __launch_bounds__(kSortThreads)
+template <int B>
+struct Bits {
+  static constexpr int value = B;
+};
+
+__global__ void __launch_bounds__(kSortThreads, 3)
 k_onesweep(const uint32_t* keys_src, const uint32_t* vals_src, uint32_t* keys_dst_out,
            uint32_t* vals_dst_out, uint32_t* keys_tmp, uint32_t* vals_tmp, SortSegment seg,
-           int pass, int passes, int digit_lo, const uint32_t* __restrict__ trivial, uint32_t key_bits,
+           int pass, int passes, int digit_lo, const uint32_t* __restrict__ varying, uint32_t key_bits,
            const uint32_t* __restrict__ hist, uint32_t* __restrict__ tile_counter,
            uint32_t* __restrict__ lookback, uint32_t max_tiles, uint32_t* __restrict__ err,
            uint32_t spin_limit, uint32_t withhold_tile0) {
@@ -167,14 +184,14 @@ k_onesweep(const uint32_t* keys_src, const uint32_t* vals_src, uint32_t* keys_ds
   __shared__ uint32_t s_scan[kWarps];
   __shared__ uint32_t s_tile;
 
-  // Trivial passes (and those below digit_lo, which are not launched) are
-  // skipped; the m remaining passes alternate between the temporary and the
+  // Passes in which no bit varies (and those below digit_lo, which are not
+  // launched) are skipped; the m remaining passes alternate between the temporary and the
   // output buffers so that the last one writes the output (with m == 0, pass
   // digit_lo runs anyway and copies: its digit is the same for every key).
   int m = 0, j = 0;
   bool skip = false;
   for (int p = 0; p < passes; ++p) {
-    const bool t = trivial[p] != 0u;
+    const bool t = varying[p] == 0u;
     if (!t) {
       if (p < pass) ++j;
       ++m;
@@ -213,30 +230,50 @@ k_onesweep(const uint32_t* keys_src, const uint32_t* vals_src, uint32_t* keys_ds
   const int shift = 8 * pass;
   const uint32_t dmask = digit_mask(key_bits, pass);
 
-  uint32_t key[kSortItems], val[kSortItems], rank[kSortItems];
+  uint32_t key[kSortItems];
   const uint32_t lt = lanemask_lt();
+  const uint32_t vary = varying[pass];
 #pragma unroll
   for (int k = 0; k < kSortItems; ++k) {
     uint32_t idx = base + warp * (32 * kSortItems) + k * 32 + lane;
-    bool valid = idx < n;
-    key[k] = valid ? keys_in[begin + idx] : 0xFFFFFFFFu;
-    val[k] = valid ? (vals_in ? vals_in[begin + idx] : begin + idx) : 0u;
+    key[k] = idx < n ? keys_in[begin + idx] : 0xFFFFFFFFu;
   }
+  // The lanes that hold the same digit, of each of the warp's rounds: a ballot
+  // per digit bit, four where the upper ones do not vary (the item sorts'
+  // depths).  match.any serialises over the distinct values of a round, about
+  // 30 of 32 random bytes: 16.7M random keys 156 -> 136 us per pass; emission
+  // keys, in runs of equal digits, 125 -> 124.  Three blocks per multiprocessor
+  // (80 registers): four at 64 registers take 145 us, and look-back over eight
+  // predecessors per round trip 191 (115 registers).
+  uint32_t rank[kSortItems / 2];  // two 16-bit ranks within the warp's digit per word
+  auto rank_keys = [&](auto bits) {
+#pragma unroll
+    for (int k = 0; k < kSortItems; ++k) {
+      const uint32_t idx = base + warp * (32 * kSortItems) + k * 32 + lane;
+      const uint32_t d = (key[k] >> shift) & dmask;
+      uint32_t peers = __ballot_sync(0xFFFFFFFFu, idx < n);
+#pragma unroll
+      for (int bit = 0; bit < bits.value; ++bit) {
+        const bool one = (d >> bit) & 1u;
+        const uint32_t ones = __ballot_sync(0xFFFFFFFFu, one);
+        peers &= one ? ones : ~ones;
+      }
+      const uint32_t cnt = s_warp_hist[warp][d];
+      __syncwarp();
+      if (idx < n && (peers & lt) == 0) s_warp_hist[warp][d] = cnt + __popc(peers);
+      __syncwarp();
+      const uint32_t rk = cnt + __popc(peers & lt);
+      rank[k / 2] = k % 2 ? rank[k / 2] | (rk << 16) : rk;
+    }
+  };
+  if (vary & 0xF0u) rank_keys(Bits<8>{});
+  else rank_keys(Bits<4>{});
+  // the values are needed after the look-back: loaded now, off its path
+  uint32_t val[kSortItems];
 #pragma unroll
   for (int k = 0; k < kSortItems; ++k) {
     uint32_t idx = base + warp * (32 * kSortItems) + k * 32 + lane;
-    bool valid = idx < n;
-    uint32_t d = (key[k] >> shift) & dmask;
-    uint32_t active = __ballot_sync(0xFFFFFFFFu, valid);
-    uint32_t peers = 0, cnt = 0;
-    if (valid) {
-      peers = __match_any_sync(active, d);
-      cnt = s_warp_hist[warp][d];
-    }
-    __syncwarp();
-    if (valid && (peers & lt) == 0) s_warp_hist[warp][d] = cnt + __popc(peers);
-    __syncwarp();
-    rank[k] = valid ? cnt + __popc(peers & lt) : 0xFFFFFFFFu;
+    val[k] = vals_in && idx < n ? vals_in[begin + idx] : begin + idx;
   }
   __syncthreads();
 
@@ -297,15 +334,17 @@ k_onesweep(const uint32_t* keys_src, const uint32_t* vals_src, uint32_t* keys_ds
   // Local scatter (stable) into shared memory.
 #pragma unroll
   for (int k = 0; k < kSortItems; ++k) {
-    if (rank[k] != 0xFFFFFFFFu) {
+    const uint32_t idx = base + warp * (32 * kSortItems) + k * 32 + lane;
+    if (idx < n) {
       uint32_t dk = (key[k] >> shift) & dmask;
-      uint32_t lp = s_block_excl[dk] + s_warp_hist[warp][dk] + rank[k];
+      uint32_t lp = s_block_excl[dk] + s_warp_hist[warp][dk] + ((rank[k / 2] >> (16 * (k % 2))) & 0xFFFFu);
       s_keys[lp] = key[k];
       s_vals[lp] = val[k];
     }
   }
   __syncthreads();
   const uint32_t cnt = min((uint32_t)kSortTile, n - base);
+#pragma unroll 4
   for (uint32_t i = tid; i < cnt; i += kSortThreads) {
     uint32_t kk = s_keys[i];
     uint32_t dk = (kk >> shift) & dmask;
@@ -381,8 +420,8 @@ cudaError_t sort_pairs_launch(const uint32_t* keys_in, const uint32_t* vals_in,
   uint32_t hist_blocks = tiles < 1024u ? tiles : 1024u;
   k_sort_hist<<<hist_blocks, kSortThreads, 0, stream>>>(keys_in, seg, passes, digit_lo, key_bits,
                                                          sc.hist, sc.lookback, sc.max_tiles);
-  uint32_t* trivial = sc.tile_counter + 8;  // cleared with the tile tickets above
-  k_sort_scan<<<passes, kRadix, 0, stream>>>(sc.hist, seg, trivial, digit_lo);
+  uint32_t* varying = sc.tile_counter + 8;  // cleared with the tile tickets above
+  k_sort_scan<<<passes, kRadix, 0, stream>>>(sc.hist, varying, digit_lo);
   // Host fault injection (SKY_FAULT=lookback:N): in the N-th fault-point sort
   // of the process, tile 0 of every digit pass withholds its look-back word
   // and the waits give up after 64 polls -- the timeout path, without a
@@ -394,7 +433,7 @@ cudaError_t sort_pairs_launch(const uint32_t* keys_in, const uint32_t* vals_in,
     k_onesweep<<<std::min<uint32_t>(tiles, (uint32_t)sm_count() * 4), kSortThreads, 0,
                  stream>>>(keys_in, vals_in, keys_out, vals_out,
                                                     sc.keys_tmp, sc.vals_tmp, seg, p, passes,
-                                                    digit_lo, trivial, key_bits, sc.hist,
+                                                    digit_lo, varying, key_bits, sc.hist,
                                                     sc.tile_counter, sc.lookback, sc.max_tiles, err,
                                                     spin_limit, inject ? 1u : 0u);
   return cudaGetLastError();
