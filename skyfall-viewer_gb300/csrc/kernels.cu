@@ -1355,18 +1355,20 @@ __global__ void __launch_bounds__(TS* TS) k_backward_exact(DevBuffers b) {
 // arithmetic is that of k_backward_exact; the per-(tile, intersection) sums
 // differ only in summation order.
 // ---------------------------------------------------------------------------
-// racc = r . acc: the residual dotted with the colour accumulated behind the
-// current splat (starting from the background), the only use of that colour.
-struct BwdPix {
-  float px, py, T, racc, r[3];
-  int hi;
+// A lane's two vertically adjacent pixels, .x the upper one.  racc = r . acc:
+// the residual dotted with the colour accumulated behind the current splat
+// (starting from the background), the only use of that colour.
+struct BwdPix2 {
+  float px;
+  float2 py, T, racc, r[3];
+  int hi[2];
 };
 
 // exp(-s) for 0 <= s <= ln(255) + 1e-3 by the ex2.approx instruction
 // (relative error below 1e-6 here, including the rounding of -s log2 e).
-SKY_DEV float exp_neg_approx(float s) {
+SKY_DEV float ex2_approx(float x) {
   float r;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(s * -1.44269504f));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
 }
 
@@ -1382,136 +1384,165 @@ SKY_DEV float sure_bound(const float4& q1, const float4& q2) {
   return q1.y > 0.9989f ? -1.0f : q2.y - 1.1e-3f;
 }
 
-// One (pixel, splat) pair of the exact backward: adds the pair's raw moments
-// to val and steps the pixel's transmittance and accumulated colour back past
-// the splat.  val[0..3] are the colour-weighted and opacity moments; since
-// a lane's two pixels share dx, val[4..6] hold sum g, sum g dy and sum g dy^2
-// (g = dL/dalpha alpha), and the entry forms g dx^2, g dx dy, g dy^2, g dx,
-// g dy from them (lane_moments).  Returns whether the splat contributes at the pixel.
+// A staged splat of the 16x16-tile backward (c twice, for both pixels' packed
+// products).
+struct __align__(16) BwdSplat {
+  float mx, a, b, smax;       // conic halved in a and c
+  float my, sure;             // sure: sure_bound
+  float2 c;
+  float opacity, red, green, blue;
+};
+
+// Both (pixel, splat) pairs of a lane and staged splat j (contributing at a
+// pixel only from jmin on): val[0..3] get the colour-weighted and opacity
+// moments; since the pixels share dx, val[4..6] get sum g, sum g dy and
+// sum g dy^2 (g = dL/dalpha alpha), and the entry forms g dx^2, g dx dy, g dy^2,
+// g dx, g dy from them.  Steps the pixels' transmittance and accumulated colour
+// back past the splat where it contributes, and returns whether it does at
+// either.
 // Which pairs contribute (alpha >= 1/255) and which are clamped (alpha >
 // 0.999) must be decided exactly as the forward decided them; the gradient
-// values only have to be accurate.  A pair with s <= s_sure (sure_bound)
-// contributes unclamped; above it, alpha comes from the fast exponential,
-// and from sky_expf (the forward's) only when it lies within 2e-6 relative of
-// either threshold, where the two could decide differently.  In both cases
-// the gradient uses the fast exponential's alpha.
-// dx = px - mx, s1 = (a/2 dx) dx (q0, q1 are staged records, conic halved)
-// and bdx = b dx belong to the pixel column and are shared by the lane's two
-// pixels.
-SKY_DEV bool bwd_pair(BwdPix& p, float dx, float s1, float bdx, const float4& q0, const float4& q1,
-                      const float4& q2, float s_sure, float val[9]) {
-  const float dy = p.py - q0.y;
-  const float s2 = (q1.x * dy) * dy;  // staged record: halved conic
-  float so2 = s1 + s2;
-  so2 = so2 + bdx * dy;
-  if (outside_smax(so2, q2.y)) return false;
-  float G = exp_neg_approx(so2);
-  float al = q1.y * G;
-  float a = al;
-  bool clamped = false;
-  if (so2 > s_sure) {
-    if (fabsf(al - MIN_ALPHA) <= 2e-6f * MIN_ALPHA || fabsf(al - MAX_ALPHA) <= 2e-6f) {
-      G = sky_expf_inrange(-so2);
-      al = q1.y * G;
-    }
-    a = fmin_(al, MAX_ALPHA);
-    if (!(a >= MIN_ALPHA)) return false;
-    clamped = al > MAX_ALPHA;  // the clamp has zero slope
+// values only have to be accurate.  A pair with s <= sure contributes
+// unclamped; above it, alpha comes from the fast exponential, and from
+// sky_expf (the forward's) only when it lies within 2e-6 relative of either
+// threshold, where the two could decide differently.  In both cases the
+// gradient uses the fast exponential's alpha.
+// There is no branch per pixel: a pair that does not contribute has alpha 0,
+// which makes its terms 0 and leaves racc and T alone (T / 1 is T: the quotient
+// multiplies by the reciprocal of 1, which is exact) -- as long as the
+// residual, the colour and their products are finite (FIN, both below
+// kBwdFinite); otherwise its operands are cleared too.  With a branch per
+// pixel, lanes of both kinds run both sides of nearly every entry.
+constexpr float kBwdFinite = 1e18f;
+template <bool FIN, bool CNT>
+SKY_DEV bool bwd_pixels(BwdPix2& p, const BwdSplat& q, int j, const int (&jmin)[2], float dx, float nz,
+                        float (&val)[7], uint32_t& n_eval, uint32_t& n_contrib) {
+  const float s1 = (q.a * dx) * dx, bdx = q.b * dx;
+  const float2 dy = make_float2(p.py.x - q.my, p.py.y - q.my);
+  const float2 s2 = mul2_rounded(__fmul2_rn(q.c, dy), dy, nz);
+  float2 s = __fadd2_rn(make_float2(s1, s1), s2);
+  s = __fadd2_rn(s, mul2_rounded(make_float2(bdx, bdx), dy, nz));
+  bool v0 = j >= jmin[0], v1 = j >= jmin[1];
+  if constexpr (CNT) n_eval += (uint32_t)v0 + (uint32_t)v1;
+  v0 = v0 && !outside_smax(s.x, q.smax);
+  v1 = v1 && !outside_smax(s.y, q.smax);
+  float2 al = make_float2(q.opacity * ex2_approx(s.x * -1.44269504f), q.opacity * ex2_approx(s.y * -1.44269504f));
+  if (!v0) al.x = 0.0f;
+  if (!v1) al.y = 0.0f;
+  float2 a = al;  // al: 0 where alpha is clamped (the clamp has zero slope)
+  if ((v0 && s.x > q.sure) || (v1 && s.y > q.sure)) {
+    auto decide = [&](bool& v, float sp, float& alp, float& ap) {
+      if (!(v && sp > q.sure)) return;
+      float t = alp;
+      if (fabsf(t - MIN_ALPHA) <= 2e-6f * MIN_ALPHA || fabsf(t - MAX_ALPHA) <= 2e-6f)
+        t = q.opacity * sky_expf_inrange(-sp);
+      ap = fmin_(t, MAX_ALPHA);
+      alp = t > MAX_ALPHA ? 0.0f : t;
+      if (!(ap >= MIN_ALPHA)) {
+        v = false;
+        ap = alp = 0.0f;
+      }
+    };
+    decide(v0, s.x, al.x, a.x);
+    decide(v1, s.y, al.y, a.y);
   }
-  const float om = 1.0f - a;  // >= 0.001 (a <= 0.999): the reference's max(1 - a, 1e-4)
-  const float Tb = __fdividef(p.T, om);
-  const float ctb = a * Tb;
+  if constexpr (CNT) n_contrib += (uint32_t)v0 + (uint32_t)v1;
+  // 1 - a >= 0.001 (a <= 0.999): the reference's max(1 - a, 1e-4)
+  const float2 Tb = make_float2(__fdividef(p.T.x, 1.0f - a.x), __fdividef(p.T.y, 1.0f - a.y));
+  const float ctb[2] = {a.x * Tb.x, a.y * Tb.y};
   // dL/dalpha = r . (colour - acc) T_before, with r . acc carried as racc
-  const float rcol = __fmaf_rn(p.r[2], q2.x, __fmaf_rn(p.r[1], q1.w, p.r[0] * q1.z));
-  const float dd = rcol - p.racc;
-  const float dLda = dd * Tb;
-  const float dl = clamped ? 0.0f : dLda;
-  const float g = dl * al;
-  const float gdy = g * dy;
-  val[0] = __fmaf_rn(p.r[0], ctb, val[0]);
-  val[1] = __fmaf_rn(p.r[1], ctb, val[1]);
-  val[2] = __fmaf_rn(p.r[2], ctb, val[2]);
-  val[3] = __fmaf_rn(dl, a, val[3]);
-  val[4] = val[4] + g;                     // sum g      (dx is the lane's)
-  val[5] = val[5] + gdy;                   // sum g dy
-  val[6] = __fmaf_rn(gdy, dy, val[6]);     // sum g dy^2
-  p.racc = __fmaf_rn(a, dd, p.racc);  // acc += a (colour - acc), dotted with r
+  float r[2][3], dd[2];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    r[0][k] = p.r[k].x;
+    r[1][k] = p.r[k].y;
+  }
+  dd[0] = __fmaf_rn(r[0][2], q.blue, __fmaf_rn(r[0][1], q.green, r[0][0] * q.red)) - p.racc.x;
+  dd[1] = __fmaf_rn(r[1][2], q.blue, __fmaf_rn(r[1][1], q.green, r[1][0] * q.red)) - p.racc.y;
+  if constexpr (!FIN) {
+    if (!v0) r[0][0] = r[0][1] = r[0][2] = dd[0] = 0.0f;
+    if (!v1) r[1][0] = r[1][1] = r[1][2] = dd[1] = 0.0f;
+  }
+  const float dl[2] = {dd[0] * Tb.x, dd[1] * Tb.y};
+  const float g[2] = {dl[0] * al.x, dl[1] * al.y};
+  const float gdy[2] = {g[0] * dy.x, g[1] * dy.y};
+#pragma unroll
+  for (int k = 0; k < 3; ++k) val[k] = __fmaf_rn(r[1][k], ctb[1], r[0][k] * ctb[0]);
+  val[3] = __fmaf_rn(dl[1], al.y, dl[0] * al.x);
+  val[4] = g[0] + g[1];
+  val[5] = gdy[0] + gdy[1];
+  val[6] = __fmaf_rn(gdy[1], dy.y, gdy[0] * dy.x);
+  // acc += a (colour - acc), dotted with r
+  p.racc = make_float2(__fmaf_rn(a.x, dd[0], p.racc.x), __fmaf_rn(a.y, dd[1], p.racc.y));
   p.T = Tb;
-  return true;
+  return v0 || v1;
 }
 
-// The nine moments of a lane from its accumulators (bwd_pair) and its dx.
-SKY_DEV void lane_moments(float val[9], float dx) {
-  const float gs = val[4], gy = val[5], gyy = val[6];
-  const float gdx = gs * dx;
-  val[4] = gdx * dx;
-  val[5] = gy * dx;
-  val[6] = gyy;
-  val[7] = gdx;
-  val[8] = gy;
+// The nine moments of a lane from its raw sums (bwd_pixels) and its dx.
+SKY_DEV void lane_moments(const float (&val)[7], float dx, float out[9]) {
+  const float gdx = val[4] * dx;
+  out[0] = val[0]; out[1] = val[1]; out[2] = val[2]; out[3] = val[3];
+  out[4] = gdx * dx;
+  out[5] = val[5] * dx;
+  out[6] = val[6];
+  out[7] = gdx;
+  out[8] = val[5];
 }
 
-// The warp's nine moment sums of an entry from the lanes' raw sums (bwd_pair's
-// val[0..6]), column first: the four lanes of a pixel column (lane & 7) share
-// dx, so the seven raw sums are added over the column (lanes l ^ 8, l ^ 16)
-// before the g sums are expanded by dx, and only then over the eight columns
-// (10 shuffles instead of 12, and the expansion once per column).  After the
-// column step a lane of row group (lane >> 3) & 3 holds two sums u0, u1
-// ({c0, c1}, {c2, g}, {o, g dy}, {g dy^2, -}) and forms u0, u1 f1, u1 f2 from
-// its factors f1 = a1 + dx (b1 + dx c1), f2 = a2 + dx b2.  On return the lane
-// with cols9_slot(lane) == k < 9 holds the warp total of lane_moments' k-th
-// value.
-struct ColFactors {
-  float a1, b1, c1, a2, b2;
-};
-// The row group's outputs u0, u1 f1, u1 f2 per case:
-SKY_DEV ColFactors col_factors(uint32_t lane) {
-  switch ((lane >> 3) & 3u) {
-    case 0: return {1.0f, 0.0f, 0.0f, 0.0f, 0.0f};  // c0, c1, (0)
-    case 1: return {0.0f, 0.0f, 1.0f, 0.0f, 1.0f};  // c2, g dx^2, g dx
-    case 2: return {0.0f, 1.0f, 0.0f, 1.0f, 0.0f};  // o, g dy dx, g dy
-    default: return {0.0f, 0.0f, 0.0f, 0.0f, 0.0f};  // g dy^2, (0), (0)
-  }
-}
-SKY_DEV int cols9_slot(uint32_t lane) {
-  if (lane & 1u) return 9;
-  const int xi = (int)((lane >> 2) & 1u) * 2 + (int)((lane >> 1) & 1u);
-  switch ((lane >> 3) & 3u) {
-    case 0: return xi == 0 ? 0 : (xi == 1 ? 1 : 9);
-    case 1: return xi == 0 ? 2 : (xi == 1 ? 4 : (xi == 2 ? 7 : 9));
-    case 2: return xi == 0 ? 3 : (xi == 1 ? 5 : (xi == 2 ? 8 : 9));
-    default: return xi == 0 ? 6 : 9;
-  }
-}
-SKY_DEV float warp_reduce_cols9(const float val[9], float dx, uint32_t lane, const ColFactors& f) {
-  const bool b4 = lane & 16u, b3 = lane & 8u, b2 = lane & 4u, b1 = lane & 2u;
-  const float v[8] = {val[0], val[1], val[2], val[4], val[3], val[5], val[6], 0.0f};
-  float w[4];
+// The warp's nine moment sums of up to kRedSlots entries at a time.  The lanes
+// leave an entry's seven raw sums (bwd_pixels) in a slot of shared memory,
+// value by value, the four rows of a pixel column (lane & 7) side by side.
+// Lane (e, c) = (lane >> 3, lane & 7) then adds column c of entry e, rows 0 and
+// 2, 1 and 3, and those; expands the g sums by the column's dx; and through
+// shared memory again lane (e, k) adds the k-th sum over the columns in the
+// order of a butterfly.  An entry costs 7 stores and a quarter of this, about
+// 25 issue slots; a shuffle butterfly per entry took about 50, most of them
+// selects on the half-rate ALU pipe.
+constexpr int kRedSlots = 4;
+static_assert(kRedSlots == 4, "eight lanes per slot: the slots fill the warp");
+SKY_DEV void reduce_slots(float* red, int ns, int j, float px, const BwdSplat* rec, float (*part)[9],
+                          uint32_t lane) {
+  const int e = (int)(lane >> 3), c = (int)(lane & 7u);
+  __syncwarp();
+  const float4* src = reinterpret_cast<const float4*>(red + e * (7 * 32)) + c;
+  float u[7];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
-    w[i] = (b4 ? v[i + 4] : v[i]) + __shfl_xor_sync(kFull, b4 ? v[i] : v[i + 4], 16);
-  float u[2];
+  for (int k = 0; k < 7; ++k) {
+    const float4 v = src[k * 8];
+    u[k] = (v.x + v.z) + (v.y + v.w);
+  }
+  const float dx = px - rec[j].mx;  // (column c's pixels: the lane's own)
+  const float x[8] = {u[0], u[1], u[2], u[3], u[4] * (dx * dx), u[5] * dx, u[6], u[4] * dx};
+  float last = u[5];
+  __syncwarp();  // the slots have been read
+  float* t = red + e * 72;
 #pragma unroll
-  for (int i = 0; i < 2; ++i)
-    u[i] = (b3 ? w[i + 2] : w[i]) + __shfl_xor_sync(kFull, b3 ? w[i] : w[i + 2], 8);
-  const float f1 = __fmaf_rn(dx, __fmaf_rn(dx, f.c1, f.b1), f.a1);
-  const float f2 = __fmaf_rn(dx, f.b2, f.a2);
-  const float x0 = u[0], x1 = u[1] * f1, x2 = u[1] * f2;
-  const float y0 = (b2 ? x2 : x0) + __shfl_xor_sync(kFull, b2 ? x0 : x2, 4);
-  const float y1 = (b2 ? 0.0f : x1) + __shfl_xor_sync(kFull, b2 ? x1 : 0.0f, 4);
-  const float z = (b1 ? y1 : y0) + __shfl_xor_sync(kFull, b1 ? y0 : y1, 2);
-  return z + __shfl_xor_sync(kFull, z, 1);
+  for (int k = 0; k < 8; ++k) t[k * 8 + c] = x[k];
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) last += __shfl_xor_sync(kFull, last, o);
+  __syncwarp();
+  const float4 lo = *reinterpret_cast<const float4*>(t + c * 8), hi = *reinterpret_cast<const float4*>(t + c * 8 + 4);
+  if (e < ns) {
+    part[j][c] = ((lo.x + hi.x) + (lo.z + hi.z)) + ((lo.y + hi.y) + (lo.w + hi.w));
+    if (c == 0) part[j][8] = last;
+  }
+  __syncwarp();  // before the slots are written again
 }
 
+// Measured: 16 views of 1M Gaussians at 1080p 7203 -> 6566 us, 4 views of 300k
+// at 720p 883 -> 807, 16k Gaussians at 256x256 150 -> 108, against a branch per
+// pixel and a shuffle butterfly per entry.  Eight blocks per multiprocessor (64
+// registers, 27 KB); nine spill (+5 %), seven lose 4 %.
 // BB: the splat-batch depth (32, 64 or 128 staged splats); the per-splat sums
 // do not depend on it.
 template <int BB, bool CNT = false>
 __global__ void __launch_bounds__(128, 8) k_backward_exact2(DevBuffers b) {
   constexpr int TS = 16, NT = 128, NW = 4, kBatch = BB;
   static_assert(BB <= NT, "one staged splat per thread and batch");
-  __shared__ float4 s_rec[kBatch * 3];
-  __shared__ uint32_t s_mask[kBatch];
+  __shared__ BwdSplat s_rec[kBatch];
+  __shared__ uint8_t s_mask[kBatch];
   __shared__ float s_part[NW][kBatch][9];
+  __shared__ __align__(16) float s_red[NW][kRedSlots * 7 * 32];
   __shared__ int s_hi[NW];
   __shared__ uint8_t s_list[NW][kBatch];
   const StepParams& sp = *b.sp;
@@ -1527,35 +1558,43 @@ __global__ void __launch_bounds__(128, 8) k_backward_exact2(DevBuffers b) {
   const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t x = tx * TS + 8u * (warp & 1u) + (lane & 7u);
   const uint32_t y0 = ty * TS + 8u * (warp >> 1) + 2u * (lane >> 3);
-  BwdPix pix[2];
+  BwdPix2 pix;
+  pix.px = (float)x + 0.5f;
+  bool infinite = false;  // a residual of this lane is, or may make a product so
+  {
+    float py[2], T[2], r[3][2], racc[2];
 #pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    BwdPix& p = pix[h];
-    const uint32_t y = y0 + (uint32_t)h;
-    p.px = (float)x + 0.5f;
-    p.py = (float)y + 0.5f;
-    p.T = 1.0f;
-    p.r[0] = p.r[1] = p.r[2] = 0.0f;
-    p.hi = (int)start - 1;
-    if (x < vi.width && y < vi.height) {
-      const size_t q = (size_t)vi.pixel_base + (size_t)y * vi.width + x;
-      const uint32_t lst = b.last[q];
-      if (lst >= start) p.hi = (int)min(lst, end - 1);
-      p.T = b.tfinal[q];
-      const float4 rs = b.residual[q];
-      p.r[0] = rs.x; p.r[1] = rs.y; p.r[2] = rs.z;
+    for (int h = 0; h < 2; ++h) {
+      const uint32_t y = y0 + (uint32_t)h;
+      py[h] = (float)y + 0.5f;
+      T[h] = 1.0f;
+      r[0][h] = r[1][h] = r[2][h] = 0.0f;
+      pix.hi[h] = (int)start - 1;
+      if (x < vi.width && y < vi.height) {
+        const size_t q = (size_t)vi.pixel_base + (size_t)y * vi.width + x;
+        const uint32_t lst = b.last[q];
+        if (lst >= start) pix.hi[h] = (int)min(lst, end - 1);
+        T[h] = b.tfinal[q];
+        const float4 rs = b.residual[q];
+        r[0][h] = rs.x; r[1][h] = rs.y; r[2][h] = rs.z;
+      }
+      racc[h] = __fmaf_rn(r[2][h], sp.bg[2], __fmaf_rn(r[1][h], sp.bg[1], r[0][h] * sp.bg[0]));
+      infinite = infinite || !(fabsf(r[0][h]) + fabsf(r[1][h]) + fabsf(r[2][h]) < kBwdFinite);
     }
-    p.racc = __fmaf_rn(p.r[2], sp.bg[2], __fmaf_rn(p.r[1], sp.bg[1], p.r[0] * sp.bg[0]));
+    pix.py = make_float2(py[0], py[1]);
+    pix.T = make_float2(T[0], T[1]);
+    pix.racc = make_float2(racc[0], racc[1]);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) pix.r[c] = make_float2(r[c][0], r[c][1]);
   }
-  int whi = max(pix[0].hi, pix[1].hi);
+  int whi = max(pix.hi[0], pix.hi[1]);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) whi = max(whi, __shfl_xor_sync(kFull, whi, o));
   if (lane == 0) s_hi[warp] = whi;
-  __syncthreads();
+  const bool finite_pixels = !__syncthreads_or(infinite);
   int hi = s_hi[0];
   for (int w = 1; w < NW; ++w) hi = max(hi, s_hi[w]);
-  const int slot = cols9_slot(lane);
-  const ColFactors cf = col_factors(lane);
+  const uint32_t red_word = 4u * (lane & 7u) + (lane >> 3);
   const uint32_t wbit = 1u << warp;
   const uint32_t lt = (1u << lane) - 1u;
   uint32_t n_eval = 0, n_contrib = 0, n_entries = 0, n_idle = 0;  // counting variant only
@@ -1567,6 +1606,7 @@ __global__ void __launch_bounds__(128, 8) k_backward_exact2(DevBuffers b) {
     // thread k stages splat k and later writes its partial: its emission
     // index is loaded here, off the write's path
     uint32_t e_mine = 0;
+    infinite = false;  // a staged colour is, or may make a product so
     for (int k = (int)tid; k < cnt; k += NT) {
       e_mine = b.vals_sorted[bhi - k];
       const size_t r = b.flatten[bhi - k];
@@ -1577,12 +1617,19 @@ __global__ void __launch_bounds__(128, 8) k_backward_exact2(DevBuffers b) {
       // every intersection up to the tile's last contributor): an 8x8 block
       // is kept when either of its two 8x4 halves is
       const uint32_t m8 = b.fmask[bhi - k];
-      s_mask[k] = ((m8 | (m8 >> 2)) & 3u) | ((((m8 >> 4) | (m8 >> 6)) & 3u) << 2);
-      // the box half-widths are only needed for the mask: the staged record
-      // carries the splat's sure bound in their place
-      stage_record(s_rec + k * 3, q0, q1, make_float4(q2.x, q2.y, sure_bound(q1, q2), q2.w));
+      s_mask[k] = (uint8_t)(((m8 | (m8 >> 2)) & 3u) | ((((m8 >> 4) | (m8 >> 6)) & 3u) << 2));
+      BwdSplat& d = s_rec[k];
+      d.mx = q0.x; d.a = 0.5f * q0.z; d.b = q0.w; d.smax = q2.y;
+      d.my = q0.y; d.sure = sure_bound(q1, q2);
+      const float ch = 0.5f * q1.x;
+      d.c = make_float2(ch, ch);
+      d.opacity = q1.y;
+      d.red = q1.z;
+      d.green = q1.w;
+      d.blue = q2.x;
+      infinite = infinite || !(q1.z + q1.w + q2.x < kBwdFinite);  // (colours are >= 0)
     }
-    __syncthreads();
+    const bool finite = !__syncthreads_or(infinite) && finite_pixels;
     uint32_t nlist = 0;
     for (int base = 0; base < cnt; base += 32) {
       const int j = base + (int)lane;
@@ -1592,43 +1639,48 @@ __global__ void __launch_bounds__(128, 8) k_backward_exact2(DevBuffers b) {
       nlist += __popc(m);
     }
     __syncwarp();
-    for (uint32_t li = 0; li < nlist; ++li) {
-      const int j = s_list[warp][li];
-      const int i = bhi - j;
-      float val[9];
-#pragma unroll
-      for (int k = 0; k < 9; ++k) val[k] = 0.0f;
-      const float4 q0 = s_rec[j * 3 + 0], q1 = s_rec[j * 3 + 1], q2 = s_rec[j * 3 + 2];
-      const float dx = pix[0].px - q0.x;
-      const float s1 = (q0.z * dx) * dx, bdx = q0.w * dx;
-      const float s_sure = q2.z;  // sure_bound, staged
-      bool contrib = false;
-      if constexpr (CNT) {
-        ++n_entries;
-        bool c0 = false, c1 = false;
-        if (i <= pix[0].hi) { ++n_eval; c0 = bwd_pair(pix[0], dx, s1, bdx, q0, q1, q2, s_sure, val); }
-        if (i <= pix[1].hi) { ++n_eval; c1 = bwd_pair(pix[1], dx, s1, bdx, q0, q1, q2, s_sure, val); }
-        n_contrib += (uint32_t)c0 + (uint32_t)c1;
-        contrib = c0 || c1;
-      } else {
-        if (i <= pix[0].hi) contrib = bwd_pair(pix[0], dx, s1, bdx, q0, q1, q2, s_sure, val);
-        if (i <= pix[1].hi) contrib = bwd_pair(pix[1], dx, s1, bdx, q0, q1, q2, s_sure, val) || contrib;
-      }
-      const uint32_t who = __ballot_sync(kFull, contrib);
-      if constexpr (CNT) n_idle += who == 0u ? 1u : 0u;
-      if (who == 0u) {
-        if (slot < 9) s_part[warp][j][slot] = 0.0f;
-      } else if ((who & (who - 1u)) == 0u) {
-        if (contrib) {
-          lane_moments(val, dx);
-#pragma unroll
-          for (int k = 0; k < 9; ++k) s_part[warp][j][k] = val[k];
+    float* const red = s_red[warp];
+    auto walk = [&](auto fin) {
+      int ns = 0, j_slot = 0;  // lane e: the entry in slot e
+      const int jmin[2] = {bhi - pix.hi[0], bhi - pix.hi[1]};  // each pixel's last contributor
+      for (uint32_t li = 0; li < nlist; ++li) {
+        const int j = s_list[warp][li];
+        const BwdSplat& q = s_rec[j];
+        const float dx = pix.px - q.mx;
+        float val[7];
+        const bool contrib =
+            bwd_pixels<fin.value, CNT>(pix, q, j, jmin, dx, b.neg_zero, val, n_eval, n_contrib);
+        const uint32_t who = __ballot_sync(kFull, contrib);
+        if constexpr (CNT) {
+          ++n_entries;
+          n_idle += who == 0u ? 1u : 0u;
         }
-      } else {
-        const float tot = warp_reduce_cols9(val, dx, lane, cf);
-        if (slot < 9) s_part[warp][j][slot] = tot;
+        if (who == 0u) {
+          if (lane < 9u) s_part[warp][j][lane] = 0.0f;
+          continue;
+        }
+        if ((who & (who - 1u)) == 0u) {
+          if (contrib) {
+            float out[9];
+            lane_moments(val, dx, out);
+#pragma unroll
+            for (int k = 0; k < 9; ++k) s_part[warp][j][k] = out[k];
+          }
+        } else {
+          float* dst = red + ns * (7 * 32) + red_word;
+#pragma unroll
+          for (int k = 0; k < 7; ++k) dst[k * 32] = val[k];
+          if ((int)lane == ns) j_slot = j;
+          if (++ns == kRedSlots) {
+            reduce_slots(red, kRedSlots, __shfl_sync(kFull, j_slot, (int)(lane >> 3)), pix.px, s_rec, s_part[warp], lane);
+            ns = 0;
+          }
+        }
       }
-    }
+      if (ns) reduce_slots(red, ns, __shfl_sync(kFull, j_slot, (int)(lane >> 3)), pix.px, s_rec, s_part[warp], lane);
+    };
+    if (finite) walk(BoolC<true>{});
+    else walk(BoolC<false>{});
     __syncthreads();
     for (int j = (int)tid; j < cnt; j += NT) {  // (j = tid: the thread that staged it)
       const int i = bhi - j;
@@ -1641,12 +1693,12 @@ __global__ void __launch_bounds__(128, 8) k_backward_exact2(DevBuffers b) {
 #pragma unroll
         for (int k = 0; k < 9; ++k) sum[k] = sum[k] + s_part[w][j][k];
       }
-      const float4 q0 = s_rec[j * 3 + 0], q1 = s_rec[j * 3 + 1];
-      const float ca = q0.z + q0.z, cc = q1.x + q1.x;  // the conic (exact doubling)
-      const float dlogit = sum[3] * (1.0f - q1.y);
+      const BwdSplat& q = s_rec[j];
+      const float ca = q.a + q.a, cc = q.c.x + q.c.x;  // the conic (exact doubling)
+      const float dlogit = sum[3] * (1.0f - q.opacity);
       const float dca = -0.5f * sum[4], dcb = -sum[5], dcc = -0.5f * sum[6];
-      const float dmx = __fmaf_rn(ca, sum[7], q0.w * sum[8]);
-      const float dmy = __fmaf_rn(q0.w, sum[7], cc * sum[8]);
+      const float dmx = __fmaf_rn(ca, sum[7], q.b * sum[8]);
+      const float dmy = __fmaf_rn(q.b, sum[7], cc * sum[8]);
       write_partial(b, e_mine, sum, dlogit, dca, dcb, dcc, dmx, dmy);
     }
   }
