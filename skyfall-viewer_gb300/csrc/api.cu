@@ -119,6 +119,9 @@ double js_literal(float f) {
   return strtod(buf, nullptr);
 }
 
+// The step status, padded so that what lies behind it is aligned.
+constexpr size_t kStatusBytes = (sizeof(DevStatus) + 255) & ~(size_t)255;
+
 enum Mode { kRender = 0, kForward = 1, kBackward = 2, kTrain = 3 };
 
 struct Buf {
@@ -167,6 +170,7 @@ struct Context {
   uint32_t view_w = 0, view_h = 0;
   SortScratch sort{};
   uint32_t icap = 0;
+  bool sized = false;  // a pass over this scene and these cameras has sized icap
   std::vector<SkyCamera> cams;
   std::vector<uint64_t> tgt_base;
   std::vector<uint8_t> tgt_set;
@@ -339,12 +343,11 @@ double position_lr(const SkyConfig& cfg, uint64_t iteration) {
 // Enqueues the pass on the context's stream.  With sizing_sync (direct
 // passes only) the intersection count is read back after the scan and the
 // buffers grown before emission, as the reference does with its host cumsum.
-int enqueue(Context* c, const Shape& sh, bool sizing_sync, uint64_t& launches, uint64_t& h2d,
-            uint64_t& d2h) {
+int enqueue(Context* c, const Shape& sh, bool sizing_sync, bool capturing, uint64_t& launches,
+            uint64_t& h2d, uint64_t& d2h) {
   cudaStream_t s = c->stream;
   DevBuffers b = make_buffers(c);
   const bool prof = sh.prof;
-  const bool capturing = !sizing_sync;
   auto mark = [&](int k) -> int {
     if (prof) CK(capturing ? cudaEventRecordWithFlags(c->ev[k], s, cudaEventRecordExternal)
                            : cudaEventRecord(c->ev[k], s));
@@ -355,8 +358,15 @@ int enqueue(Context* c, const Shape& sh, bool sizing_sync, uint64_t& launches, u
   h2d = sizeof(StepParams);
   d2h = 0;
   CK(cudaMemcpyAsync(c->d_sp.p, c->h_sp, sizeof(StepParams), cudaMemcpyHostToDevice, s));
-  CK(cudaMemsetAsync(c->d_st.p, 0, sizeof(DevStatus), s));
+  // one clear: the status and, behind it, the digit counts and tickets of the
+  // step's sorts (an item and a tile sort per group)
+  CK(cudaMemsetAsync(c->d_st.p, 0, kStatusBytes + (size_t)2 * sh.ngroups * kSortClearBytes, s));
   DevStatus* dst = (DevStatus*)c->d_st.p;
+  auto scratch = [&](SortScratch sc, uint32_t k) {  // with the step's k-th cleared block
+    sc.hist = (uint32_t*)((char*)c->d_st.p + kStatusBytes + (size_t)k * kSortClearBytes);
+    sc.tile_counter = sc.hist + kMaxPasses * kRadix;
+    return sc;
+  };
   TRY(mark(0));
   launch_preprocess(b, sh.n, sh.nv, s);
   TRY(mark(1));
@@ -369,13 +379,11 @@ int enqueue(Context* c, const Shape& sh, bool sizing_sync, uint64_t& launches, u
       // bounds = {item_begin, item_end} of the group, in device memory
       SortSegment seg{&d_sp->groups[g].item_begin, 0};
       CK(sort_pairs_launch(b.ikeys, nullptr, (uint32_t*)c->ikeys_sorted.p, b.perm, seg,
-                           (uint32_t)items, 16, c->isort, &dst->error, s, 0, true));
+                           (uint32_t)items, 16, scratch(c->isort, 2 * g), &dst->error, s, 0, true, true));
       launches += 4;
     }
   }
-  launch_scan(b, (uint32_t)items, s);
-  launch_group_bounds(b, s);
-  launches += 5;
+  launches += 1 + launch_scan(b, (uint32_t)items, true, s);
   if (sizing_sync) {
     d2h += sizeof(DevStatus);
     CK(cudaMemcpyAsync(c->h_st, c->d_st.p, sizeof(DevStatus), cudaMemcpyDeviceToHost, s));
@@ -403,7 +411,7 @@ int enqueue(Context* c, const Shape& sh, bool sizing_sync, uint64_t& launches, u
     // the tile field (digits 2 and 3) alone gives the full key order
     SortSegment seg{&dst->group_bounds[g][0], 0};
     CK(sort_pairs_launch(b.keys, nullptr, b.keys_sorted, b.vals_sorted, seg, c->icap, sh.key_bits[g],
-                         c->sort, &dst->error, s, 2, true));
+                         scratch(c->sort, 2 * g + 1), &dst->error, s, 2, true, true));
     launches += 2 + (sh.key_bits[g] + 7) / 8 - 2;
   }
   TRY(mark(4));
@@ -411,8 +419,8 @@ int enqueue(Context* c, const Shape& sh, bool sizing_sync, uint64_t& launches, u
   TRY(mark(5));
   launch_forward(b, sh.max_tiles, c->cfg.tile_size, sh.fwd_batch, sh.ssim, sh.nv, sh.max_view_px,
                  sh.count, s);
-  if (sh.with_loss) launch_loss_final(b, s);
-  launches += 4 + (sh.with_loss ? 1 : 0) + (sh.ssim ? 1 : 0);
+  if (sh.with_loss) launch_loss_final(b, sh.max_tiles, s);
+  launches += 3 + (sh.with_loss ? 1 : 0) + (sh.ssim ? 1 : 0);
   TRY(mark(6));
   if (sh.mode >= kBackward) {
     if (sh.ref) CK(cudaMemsetAsync(c->gsum54.p, 0, items * 54 * 8, s));
@@ -530,7 +538,7 @@ int run_views(Context* c, const uint32_t* cams, uint32_t nv, Mode mode, SkyStepS
   c->isort = sort_scratch_carve(c->isort_mem.p, (uint32_t)items);
   TRY(dev_alloc(c, c->block_sums, (scan_block_count((uint32_t)items) + 1) * 4));
   TRY(dev_alloc(c, c->offsets, (tile_cap + 1) * 4));
-  TRY(dev_alloc(c, c->loss_partials, (tile_cap + 1) * 8));
+  TRY(dev_alloc(c, c->loss_partials, loss_partial_count(tile_cap) * 8));
   TRY(dev_alloc(c, c->color, pix_cap * 16));
   TRY(dev_alloc(c, c->alpha, pix_cap * 4));
   TRY(dev_alloc(c, c->tfinal, pix_cap * 4));
@@ -628,14 +636,19 @@ int run_views(Context* c, const uint32_t* cams, uint32_t nv, Mode mode, SkyStepS
   for (int attempt = 0;; ++attempt) {
     sh.icap = c->icap;
     sp.icap = c->icap;
+    // a direct pass reads its intersection count back after the scan only
+    // while the capacity is unknown; later ones check it on the device, as a
+    // graph replay does, and run again, sized, if it did not suffice (the
+    // read-back left the GPU idle for about 25 us)
+    const bool sizing = !graph && (!c->sized || attempt > 0);
     if (!graph) {
-      TRY(enqueue(c, sh, true, launches, h2d, d2h));
+      TRY(enqueue(c, sh, sizing, false, launches, h2d, d2h));
     } else {
       if (!c->gvalid || !c->gshape.same(sh)) {
         drop_graph(c);
         CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
         uint64_t l = 0, gi = 0, go = 0;
-        int rc = enqueue(c, sh, false, l, gi, go);
+        int rc = enqueue(c, sh, false, true, l, gi, go);
         cudaGraph_t g = nullptr;
         cudaError_t e = cudaStreamEndCapture(s, &g);
         if (rc != SKY_OK) {
@@ -663,8 +676,9 @@ int run_views(Context* c, const uint32_t* cams, uint32_t nv, Mode mode, SkyStepS
     c->launches += launches;
     c->step_h2d += h2d;
     c->step_d2h += d2h;
-    if (graph && (c->h_st->error & SKY_DEVERR_CAPACITY) && attempt < 3) {
-      // the failed replay changed no parameter: grow, re-capture, run again
+    if (!sizing && (c->h_st->error & SKY_DEVERR_CAPACITY) && attempt < 3) {
+      // the failed pass changed no parameter: grow (a replay is captured
+      // again), run again
       TRY(ensure_isect(c, c->h_st->total_isect));
       drop_graph(c);
       continue;
@@ -688,6 +702,7 @@ int run_views(Context* c, const uint32_t* cams, uint32_t nv, Mode mode, SkyStepS
                 "tile counts, or the tile ranges met unsorted keys");
   if (c->h_st->error & SKY_DEVERR_CAPACITY)
     return fail(SKY_ERR_CAPACITY, "intersection capacity exceeded");
+  c->sized = true;
   c->last_views.assign(cams, cams + nv);
   c->last_items = (uint32_t)items;
   c->last_tiles = (uint32_t)tile_total;
@@ -854,7 +869,7 @@ int scan_flags(Context* c, const uint32_t* flags, uint32_t* out, uint32_t n) {
   sb.counts = (uint32_t*)flags;
   sb.cumsum = out;
   sb.block_sums = bs.as<uint32_t>();
-  launch_scan(sb, n, c->stream);
+  launch_scan(sb, n, false, c->stream);
   c->launches += 3;
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(c->stream));
@@ -1161,7 +1176,7 @@ int sky_create(const SkyConfig* cfg, void** out) {
   e = cudaMallocHost(&c->h_st, sizeof(DevStatus));
   if (e != cudaSuccess) return bail(fail(SKY_ERR_OOM, "pinned alloc: %s", cudaGetErrorString(e)));
   if ((rc = dev_alloc(c, c->d_sp, sizeof(StepParams))) != SKY_OK) return bail(rc);
-  if ((rc = dev_alloc(c, c->d_st, sizeof(DevStatus))) != SKY_OK) return bail(rc);
+  if ((rc = dev_alloc(c, c->d_st, kStatusBytes + (size_t)2 * kMaxGroups * kSortClearBytes)) != SKY_OK) return bail(rc);
   *out = c;
   return SKY_OK;
 }
@@ -1249,6 +1264,7 @@ static int load_planes(Context* c, uint32_t n) {
   c->adam_steps = 0;
   c->adam_views = 0;
   c->fwd_ready = false;
+  c->sized = false;
   c->scores_valid = false;
   c->scores_n = 0;
   TRY(reset_stats(c));
@@ -1538,6 +1554,7 @@ int sky_set_cameras(void* p, const SkyCamera* cams, uint32_t n) {
   c->tgt_set.assign(n, 0);
   c->targets_px = 0;
   c->fwd_ready = false;
+  c->sized = false;
   return SKY_OK;
 }
 
@@ -2018,8 +2035,7 @@ int sky_view_render(void* p, const SkyCamera* cam, const SkyViewSettings* vs, fl
   sb.counts = (uint32_t*)c->v_csorted.p;
   sb.cumsum = (uint32_t*)c->v_cum.p;
   sb.block_sums = (uint32_t*)c->v_bsums.p;
-  launch_scan(sb, n, s);
-  c->launches += 8;
+  c->launches += 5 + launch_scan(sb, n, false, s);
   // per quad-tile pair: emit in depth order, stable sort by tile, ranges
   if (I > 0) {
     TRY(dev_alloc(c, c->v_tkeys, (size_t)I * 4));

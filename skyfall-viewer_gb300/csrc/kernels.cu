@@ -334,12 +334,25 @@ SKY_DEV uint32_t block_excl_scan(uint32_t x, uint32_t* s_warp, uint32_t& total) 
   return y - x + add;
 }
 
-// Count at scan position i: the counts are scanned in perm order when a
-// permutation is given, read from the sorted item keys (which carry them up
-// to 0xFFFF; larger ones are gathered).
-SKY_DEV uint32_t scan_count(const DevBuffers& b, uint32_t i) {
-  if (!b.perm) return b.counts[i];
-  const uint32_t c = b.ikeys_sorted[i] >> 16;
+// The counts at scan positions [i, i + 4) (i a multiple of 4): scanned in perm
+// order when a permutation is given, read from the sorted item keys (which
+// carry them up to 0xFFFF; larger ones are gathered).
+SKY_DEV uint4 scan_counts4(const DevBuffers& b, uint32_t i, uint32_t n_items) {
+  const uint32_t* src = b.perm ? b.ikeys_sorted : b.counts;
+  uint4 c;
+  if (i + 4u <= n_items) {
+    c = *reinterpret_cast<const uint4*>(src + i);
+  } else {
+    c.x = i < n_items ? src[i] : 0u;
+    c.y = i + 1u < n_items ? src[i + 1u] : 0u;
+    c.z = i + 2u < n_items ? src[i + 2u] : 0u;
+    c.w = 0u;
+  }
+  return c;
+}
+SKY_DEV uint32_t scan_count(const DevBuffers& b, uint32_t word, uint32_t i) {
+  if (!b.perm) return word;
+  const uint32_t c = word >> 16;
   return c < 0xFFFFu ? c : b.counts[b.perm[i]];
 }
 
@@ -347,14 +360,21 @@ SKY_DEV uint32_t scan_count(const DevBuffers& b, uint32_t i) {
 // the permutation may hold stale words, which must not be used as indices.
 SKY_DEV bool scan_skipped(const DevBuffers& b) { return b.status && capacity_failed(b.status); }
 
+// (all of a thread's loads are issued before the first is used: at 16k items
+// a loop of one load and one add took 10 us for four blocks)
 __global__ void __launch_bounds__(kScanThreads) k_scan_reduce(DevBuffers b, uint32_t n_items) {
   __shared__ uint32_t s_warp[kScanThreads / 32];
   if (scan_skipped(b)) return;
-  const uint32_t base = blockIdx.x * kScanTile;
+  const uint32_t base = blockIdx.x * kScanTile + 4u * threadIdx.x;
+  uint4 w[kScanItems / 4];
+#pragma unroll
+  for (int k = 0; k < kScanItems / 4; ++k) w[k] = scan_counts4(b, base + 4u * kScanThreads * k, n_items);
   uint32_t sum = 0;
-  for (int k = 0; k < kScanItems; ++k) {
-    uint32_t i = base + k * kScanThreads + threadIdx.x;
-    if (i < n_items) sum += scan_count(b, i);
+#pragma unroll
+  for (int k = 0; k < kScanItems / 4; ++k) {
+    const uint32_t i = base + 4u * kScanThreads * k;
+    sum += scan_count(b, w[k].x, i) + scan_count(b, w[k].y, i + 1u) + scan_count(b, w[k].z, i + 2u) +
+           scan_count(b, w[k].w, i + 3u);
   }
   uint32_t total;
   block_excl_scan(sum, s_warp, total);
@@ -375,35 +395,100 @@ __global__ void __launch_bounds__(1024) k_scan_blocks(DevBuffers b, uint32_t nbl
   }
 }
 
-__global__ void __launch_bounds__(kScanThreads) k_scan_final(DevBuffers b, uint32_t n_items) {
+// own_prefix: each block adds the sums of the blocks before it itself (a
+// launch less; up to kScanOwnPrefix blocks, 16 sums per thread).  bounds: a
+// step's scan, which also writes the sort groups' bounds and the capacity
+// check (b.status zeroed before, so that after an earlier error every group
+// is empty).
+constexpr uint32_t kScanOwnPrefix = 4096;
+__global__ void __launch_bounds__(kScanThreads) k_scan_final(DevBuffers b, uint32_t n_items, bool own_prefix,
+                                                             bool bounds) {
   __shared__ uint32_t s_warp[kScanThreads / 32];
   if (scan_skipped(b)) return;
   const uint32_t base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
+  uint4 w[kScanItems / 4], pv[kScanItems / 4];
+#pragma unroll
+  for (int k = 0; k < kScanItems / 4; ++k) w[k] = scan_counts4(b, base + 4u * k, n_items);
+  // the items of the scatter below, loaded ahead: a load after a store
+  // would wait for it (the arrays may alias as far as the compiler knows)
+#pragma unroll
+  for (int k = 0; k < kScanItems / 4; ++k) {
+    const uint32_t i = base + 4u * k;
+    pv[k] = make_uint4(0u, 0u, 0u, 0u);
+    if (b.perm) {
+      if (i + 4u <= n_items) {
+        pv[k] = *reinterpret_cast<const uint4*>(b.perm + i);
+      } else {
+        if (i < n_items) pv[k].x = b.perm[i];
+        if (i + 1u < n_items) pv[k].y = b.perm[i + 1u];
+        if (i + 2u < n_items) pv[k].z = b.perm[i + 2u];
+      }
+    }
+  }
+  uint32_t before = 0;
+  if (own_prefix) {
+    uint32_t part = 0;
+    for (uint32_t k = threadIdx.x; k < blockIdx.x; k += kScanThreads) part += b.block_sums[k];
+    block_excl_scan(part, s_warp, before);
+  } else {
+    before = b.block_sums[blockIdx.x];
+  }
   uint32_t v[kScanItems], pi[kScanItems];
   uint32_t sum = 0;
 #pragma unroll
   for (int k = 0; k < kScanItems; ++k) {
-    uint32_t i = base + k;
-    v[k] = i < n_items ? scan_count(b, i) : 0u;
-    // the items of the scatter below, loaded ahead: a load after a store
-    // would wait for it (the arrays may alias as far as the compiler knows)
-    pi[k] = (b.perm && i < n_items) ? b.perm[i] : 0u;
+    const uint32_t word = k % 4 == 0 ? w[k / 4].x : k % 4 == 1 ? w[k / 4].y : k % 4 == 2 ? w[k / 4].z : w[k / 4].w;
+    pi[k] = k % 4 == 0 ? pv[k / 4].x : k % 4 == 1 ? pv[k / 4].y : k % 4 == 2 ? pv[k / 4].z : pv[k / 4].w;
+    v[k] = scan_count(b, word, base + k);
     sum += v[k];
   }
   uint32_t total;
-  uint32_t run = block_excl_scan(sum, s_warp, total) + b.block_sums[blockIdx.x];
+  uint32_t run = block_excl_scan(sum, s_warp, total) + before;
 #pragma unroll
   for (int k = 0; k < kScanItems; ++k) {
     run += v[k];
-    uint32_t i = base + k;
-    if (i < n_items) {
-      b.cumsum[i] = run;
-      if (b.perm) b.item_end[pi[k]] = run;
+    v[k] = run;
+  }
+#pragma unroll
+  for (int k = 0; k < kScanItems; k += 4) {
+    const uint32_t i = base + k;
+    if (i + 4u <= n_items) {
+      *reinterpret_cast<uint4*>(b.cumsum + i) = make_uint4(v[k], v[k + 1], v[k + 2], v[k + 3]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (i + j < n_items) b.cumsum[i + j] = v[k + j];
     }
+  }
+  if (b.perm) {
+#pragma unroll
+    for (int k = 0; k < kScanItems; ++k)
+      if (base + k < n_items) b.item_end[pi[k]] = v[k];
+  }
+  if (!bounds) return;
+  const StepParams& sp = *b.sp;
+  auto clamped = [&](uint32_t end, uint32_t x) {  // x = cumsum[end - 1] when that item is this thread's
+    if (end == n_items) {
+      b.status->total_isect = x;
+      if (x > sp.icap) atomicOr(&b.status->error, SKY_DEVERR_CAPACITY);
+    }
+    return min(x, sp.icap);
+  };
+  for (uint32_t g = 0; g < sp.num_groups; ++g) {
+    const uint32_t end = sp.groups[g].item_end;
+    if (end <= base || end > base + kScanItems) continue;
+    uint32_t x = 0;
+#pragma unroll
+    for (int k = 0; k < kScanItems; ++k)
+      if (base + k + 1u == end) x = v[k];
+    x = clamped(end, x);
+    b.status->group_bounds[g][1] = x;
+    if (g + 1u < sp.num_groups) b.status->group_bounds[g + 1u][0] = x;
   }
 }
 
-// Group bounds of the sort segments and the capacity check.
+// Group bounds of the sort segments and the capacity check, again after the
+// buffers have grown (k_scan_final writes them first).
 // After an earlier error (the item sort gave up, so the scan was skipped)
 // the step has no intersections: every group is empty.
 __global__ void k_group_bounds(DevBuffers b) {
@@ -544,7 +629,11 @@ __global__ void __launch_bounds__(256) k_ranges(DevBuffers b) {
   const bool resolve = sp.bwd_mode != 0;
   for (int g = 0; g < ng; ++g) {
     const uint32_t gb = s_gb[g][0], ge = s_gb[g][1], tb = s_gt[g][0], te = s_gt[g][1];
-    if (gb >= ge) continue;  // empty: k_ranges_empty
+    if (gb >= ge) {  // empty: every tile's range, and offsets[tile_end], start at the bound
+      for (uint32_t u = tb + blockIdx.x * blockDim.x + threadIdx.x; u <= te; u += gridDim.x * blockDim.x)
+        b.offsets[u] = gb;
+      continue;
+    }
     const uint32_t c_lo = gb / 4u, c_hi = (ge + 3u) / 4u;
     for (uint32_t c = c_lo + blockIdx.x * blockDim.x + threadIdx.x; c < c_hi;
          c += gridDim.x * blockDim.x) {
@@ -591,20 +680,6 @@ __global__ void __launch_bounds__(256) k_flatten_fill(DevBuffers b, uint32_t tot
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
     const uint32_t e = b.vals_sorted[i];
     if (e < total) b.flatten[i] = b.rec_of[e];
-  }
-}
-
-// Empty groups: every tile's range, and the group's offsets[tile_end], start
-// at the group's bound.
-__global__ void k_ranges_empty(DevBuffers b) {
-  const StepParams& sp = *b.sp;
-  if (capacity_failed(b.status)) return;
-  for (uint32_t g = 0; g < sp.num_groups; ++g) {
-    const uint32_t gb = b.status->group_bounds[g][0], ge = b.status->group_bounds[g][1];
-    if (gb != ge) continue;
-    const GroupInfo& gi = sp.groups[g];
-    for (uint32_t u = gi.tile_begin + threadIdx.x; u <= gi.tile_end; u += blockDim.x)
-      b.offsets[u] = gb;
   }
 }
 
@@ -1086,33 +1161,44 @@ __global__ void __launch_bounds__(256, 4) k_ssim(DevBuffers b) {
   }
 }
 
-__global__ void __launch_bounds__(1024) k_loss_final(DevBuffers b) {
-  __shared__ double s[32];
+constexpr int kLossThreads = 256, kLossAhead = 16;
+constexpr uint32_t kLossSlice = kLossThreads * kLossAhead;  // tiles
+__global__ void __launch_bounds__(kLossThreads) k_loss_final(DevBuffers b) {
+  __shared__ double s[kLossThreads / 32];
+  __shared__ uint32_t s_last;
   const StepParams& sp = *b.sp;
-  double acc = 0.0;
-  // fixed assignment of tiles to threads, then a fixed tree; a thread's
-  // partials are loaded 16 at a time and added in order (one load, one add
-  // after another would wait on every load)
-  constexpr uint32_t kAhead = 16;
-  const uint32_t nt = sp.num_tiles, step = blockDim.x;
-  uint32_t t = threadIdx.x;
-  for (; t + (kAhead - 1) * step < nt; t += kAhead * step) {
-    double v[kAhead];
+  const uint32_t nt = sp.num_tiles, slices = (nt + kLossSlice - 1) / kLossSlice;
+  double* const sums = b.loss_partials + nt;
+  for (uint32_t sl = blockIdx.x; sl < slices; sl += gridDim.x) {
+    double v[kLossAhead], acc = 0.0;
 #pragma unroll
-    for (uint32_t k = 0; k < kAhead; ++k) v[k] = b.loss_partials[t + k * step];
+    for (int k = 0; k < kLossAhead; ++k) {
+      const uint32_t t = sl * kLossSlice + (uint32_t)k * kLossThreads + threadIdx.x;
+      v[k] = t < nt ? b.loss_partials[t] : 0.0;
+    }
 #pragma unroll
-    for (uint32_t k = 0; k < kAhead; ++k) acc += v[k];
+    for (int k = 0; k < kLossAhead; ++k) acc += v[k];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(kFull, acc, o);
+    if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = acc;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      double t = 0.0;
+      for (int w = 0; w < kLossThreads / 32; ++w) t += s[w];
+      sums[sl] = t;
+      __threadfence();
+    }
+    __syncthreads();
   }
-  for (; t < nt; t += step) acc += b.loss_partials[t];
+  if (threadIdx.x == 0) s_last = atomicAdd(&b.status->loss_blocks, 1u) == gridDim.x - 1u;
+  __syncthreads();
+  if (!s_last || threadIdx.x >= 32) return;
+  __threadfence();
+  double acc = 0.0;
+  for (uint32_t sl = threadIdx.x; sl < slices; sl += 32) acc += *(volatile const double*)&sums[sl];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(kFull, acc, o);
-  if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = acc;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += s[w];
-    b.status->loss = t;
-  }
+  if (threadIdx.x == 0) b.status->loss = acc;
 }
 
 // ---------------------------------------------------------------------------
@@ -2586,12 +2672,14 @@ void launch_preprocess(const DevBuffers& b, uint32_t n, uint32_t views, cudaStre
   k_preprocess<<<(n + kPrepThreads - 1) / kPrepThreads, kPrepThreads, views * sizeof(ViewInfo), s>>>(b);
 }
 
-void launch_scan(const DevBuffers& b, uint32_t n_items, cudaStream_t s) {
+int launch_scan(const DevBuffers& b, uint32_t n_items, bool step, cudaStream_t s) {
   const uint32_t nb = (n_items + kScanTile - 1) / kScanTile;
-  if (nb == 0) return;
+  if (nb == 0) return 0;
+  const bool own_prefix = nb <= kScanOwnPrefix;
   k_scan_reduce<<<nb, kScanThreads, 0, s>>>(b, n_items);
-  k_scan_blocks<<<1, 1024, 0, s>>>(b, nb);
-  k_scan_final<<<nb, kScanThreads, 0, s>>>(b, n_items);
+  if (!own_prefix) k_scan_blocks<<<1, 1024, 0, s>>>(b, nb);
+  k_scan_final<<<nb, kScanThreads, 0, s>>>(b, n_items, own_prefix, step);
+  return own_prefix ? 2 : 3;
 }
 
 uint32_t scan_block_count(uint32_t n_items) { return (n_items + kScanTile - 1) / kScanTile; }
@@ -2604,11 +2692,8 @@ void launch_emit(const DevBuffers& b, uint32_t n, uint32_t views, cudaStream_t s
 }
 
 void launch_ranges(const DevBuffers& b, uint32_t icap, cudaStream_t s) {
-  if (icap) {
-    const uint32_t blocks = min((icap / 4 + 255) / 256 + 1, (uint32_t)sm_count() * 8);
-    k_ranges<<<blocks, 256, 0, s>>>(b);
-  }
-  k_ranges_empty<<<1, 256, 0, s>>>(b);
+  const uint32_t blocks = min((icap / 4 + 255) / 256 + 1, (uint32_t)sm_count() * 8);
+  k_ranges<<<blocks, 256, 0, s>>>(b);
 }
 
 // Zeroes the partials the last backward did not write (unflagged), for a
@@ -2661,7 +2746,11 @@ void launch_forward(const DevBuffers& b, uint32_t max_tiles, uint32_t ts, uint32
   }
 }
 
-void launch_loss_final(const DevBuffers& b, cudaStream_t s) { k_loss_final<<<1, 1024, 0, s>>>(b); }
+size_t loss_partial_count(uint64_t tiles) { return (size_t)(tiles + tiles / kLossSlice + 1); }
+
+void launch_loss_final(const DevBuffers& b, uint32_t max_tiles, cudaStream_t s) {
+  k_loss_final<<<std::max(1u, std::min((max_tiles + kLossSlice - 1) / kLossSlice, 64u)), kLossThreads, 0, s>>>(b);
+}
 
 void launch_backward(const DevBuffers& b, uint32_t max_tiles, uint32_t ts, uint32_t bb, bool ref,
                      bool count, cudaStream_t s) {

@@ -7,7 +7,9 @@
 namespace sky {
 
 void launch_preprocess(const DevBuffers& b, uint32_t n, uint32_t views, cudaStream_t s);
-void launch_scan(const DevBuffers& b, uint32_t n_items, cudaStream_t s);
+// step: the scan of a step's items, which also writes the sort groups' bounds
+// and checks the capacity.  Returns the number of kernels launched.
+int launch_scan(const DevBuffers& b, uint32_t n_items, bool step, cudaStream_t s);
 uint32_t scan_block_count(uint32_t n_items);
 void launch_group_bounds(const DevBuffers& b, cudaStream_t s);
 void launch_emit(const DevBuffers& b, uint32_t n, uint32_t views, cudaStream_t s);
@@ -24,7 +26,9 @@ constexpr uint32_t kBwdBatch16 = 64;  // default backward depth for 16x16 tiles
 // only; other shapes launch the plain kernels and count nothing).
 void launch_forward(const DevBuffers& b, uint32_t max_tiles, uint32_t ts, uint32_t fb, bool ssim,
                     uint32_t views, uint32_t max_view_pixels, bool count, cudaStream_t s);
-void launch_loss_final(const DevBuffers& b, cudaStream_t s);
+// Doubles of b.loss_partials for a step of `tiles` tiles.
+size_t loss_partial_count(uint64_t tiles);
+void launch_loss_final(const DevBuffers& b, uint32_t max_tiles, cudaStream_t s);
 void launch_backward(const DevBuffers& b, uint32_t max_tiles, uint32_t ts, uint32_t bb, bool ref,
                      bool count, cudaStream_t s);
 // Training steps of at most kFewViews views in the exact backward mode hand the

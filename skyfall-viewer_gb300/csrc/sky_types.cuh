@@ -60,7 +60,8 @@ struct StepParams {
 struct DevStatus {
   uint32_t error;        // SKY_DEVERR_* bits
   uint32_t total_isect;  // intersections of the step (unclamped)
-  uint32_t pad[2];
+  uint32_t loss_blocks;  // blocks of the loss total that are done
+  uint32_t pad;
   uint32_t group_bounds[kMaxGroups][2];  // [begin, end) clamped to capacity
   double loss;
   double pad2;
@@ -107,7 +108,7 @@ struct DevBuffers {
   int32_t* tile_grads;    // reference mode: 54 per sorted intersection
   long long* gsum54;      // reference mode: 54 per item
   uint32_t* offsets;      // tile ranges, num_tiles + 1
-  double* loss_partials;  // per tile
+  double* loss_partials;  // per tile, then per slice of tiles
   float4* color;
   float* alpha;
   float* tfinal;      // final transmittance, product of (1 - alpha)

@@ -393,8 +393,8 @@ SortScratch sort_scratch_carve(void* base, uint32_t max_n) {
     return r;
   };
   SortScratch s;
-  s.hist = (uint32_t*)take(kMaxPasses * kRadix * 4);
-  s.tile_counter = (uint32_t*)take(256);
+  s.hist = (uint32_t*)take(kSortClearBytes);
+  s.tile_counter = s.hist + kMaxPasses * kRadix;
   s.lookback = (uint32_t*)take((size_t)kMaxPasses * tiles * kRadix * 4);
   s.keys_tmp = (uint32_t*)take((size_t)(max_n + 64) * 4);
   s.vals_tmp = (uint32_t*)take((size_t)(max_n + 64) * 4);
@@ -406,15 +406,15 @@ cudaError_t sort_pairs_launch(const uint32_t* keys_in, const uint32_t* vals_in,
                               uint32_t* keys_out, uint32_t* vals_out, SortSegment seg,
                               uint32_t max_n, uint32_t key_bits, const SortScratch& sc,
                               uint32_t* err, cudaStream_t stream, int digit_lo,
-                              bool fault_point) {
+                              bool fault_point, bool cleared) {
   if (key_bits == 0) key_bits = 1;
   if (key_bits > 32) key_bits = 32;
   const int passes = (int)((key_bits + 7) / 8);
   digit_lo = std::max(0, std::min(digit_lo, passes - 1));
-  cudaError_t e = cudaMemsetAsync(sc.hist, 0, kMaxPasses * kRadix * 4, stream);
-  if (e != cudaSuccess) return e;
-  e = cudaMemsetAsync(sc.tile_counter, 0, 256, stream);
-  if (e != cudaSuccess) return e;
+  if (!cleared) {
+    cudaError_t e = cudaMemsetAsync(sc.hist, 0, kSortClearBytes, stream);
+    if (e != cudaSuccess) return e;
+  }
   uint32_t tiles = (max_n + kSortTile - 1) / kSortTile;
   if (tiles == 0) tiles = 1;
   uint32_t hist_blocks = tiles < 1024u ? tiles : 1024u;

@@ -31,9 +31,12 @@ constexpr uint32_t SKY_DEVERR_SORT_TIMEOUT = 2u;
 // tile ranges met sorted keys out of order.  Later kernels of the step skip.
 constexpr uint32_t SKY_DEVERR_LISTS = 4u;
 
+// Cleared before every sort: the digit counts and, behind them, the tickets.
+constexpr size_t kSortClearBytes = (size_t)kMaxPasses * kRadix * 4 + 256;
+
 struct SortScratch {
   uint32_t* hist;          // kMaxPasses * 256 digit counts, then exclusive offsets
-  uint32_t* tile_counter;  // kMaxPasses tile tickets
+  uint32_t* tile_counter;  // kMaxPasses tile tickets (256 bytes, right behind hist)
   uint32_t* lookback;      // kMaxPasses * max_tiles * 256 status words
   uint32_t* keys_tmp;      // ping-pong
   uint32_t* vals_tmp;
@@ -57,11 +60,12 @@ struct SortSegment {
 // fault_point: the sort counts for SKY_FAULT=lookback:N (host fault
 // injection, used by tests); only callers whose later kernels check the
 // error word before indexing with the sort's output pass true.
+// cleared: the caller has zeroed the kSortClearBytes at sc.hist.
 cudaError_t sort_pairs_launch(const uint32_t* keys_in, const uint32_t* vals_in,
                               uint32_t* keys_out, uint32_t* vals_out, SortSegment seg,
                               uint32_t max_n, uint32_t key_bits, const SortScratch& sc,
                               uint32_t* err, cudaStream_t stream, int digit_lo = 0,
-                              bool fault_point = false);
+                              bool fault_point = false, bool cleared = false);
 
 // Host fault injection (SKY_FAULT=lookback:N, api.cu): true for the N-th
 // fault-point sort launched outside graph capture in the process.  Without
