@@ -166,7 +166,7 @@ struct Context {
   uint32_t densify_runs = 0, prune_runs = 0;
   // headless viewer frame
   Buf v_splats, v_keys, v_counts, v_rects, v_order, v_ksorted, v_cum, v_csorted, v_bsums, v_misc,
-      v_tkeys, v_gidx, v_tkeys_s, v_gidx_s, v_offsets, v_rgba, v_sort;
+      v_tkeys, v_gidx, v_tkeys_s, v_gidx_s, v_offsets, v_rgba, v_rgba8, v_sort;
   uint32_t view_w = 0, view_h = 0;
   SortScratch sort{};
   uint32_t icap = 0;
@@ -1196,7 +1196,7 @@ int sky_destroy(void* p) {
                 &c->metric_part, &c->metric_stats, &c->v_splats, &c->v_keys, &c->v_counts,
                 &c->v_rects, &c->v_order, &c->v_ksorted, &c->v_cum, &c->v_csorted, &c->v_bsums,
                 &c->v_misc, &c->v_tkeys, &c->v_gidx, &c->v_tkeys_s, &c->v_gidx_s, &c->v_offsets,
-                &c->v_rgba, &c->v_sort, &c->item_sums, &c->sh_items};
+                &c->v_rgba, &c->v_rgba8, &c->v_sort, &c->item_sums, &c->sh_items};
   for (Buf* b : all) dev_free(c, *b);
   drop_graph(c);
   for (int k = 0; k <= SKY_NUM_STAGES; ++k)
@@ -2014,6 +2014,7 @@ int sky_view_render(void* p, const SkyCamera* cam, const SkyViewSettings* vs, fl
   TRY(dev_alloc(c, c->v_misc, 64));
   TRY(dev_alloc(c, c->v_offsets, ((size_t)tiles + 1) * 4));
   TRY(dev_alloc(c, c->v_rgba, px * 16));
+  if (rgba8) TRY(dev_alloc(c, c->v_rgba8, px * 4));
   unsigned long long* d_total = (unsigned long long*)c->v_misc.p;
   uint32_t* d_err = (uint32_t*)((char*)c->v_misc.p + 8);
   CK(cudaMemsetAsync(c->v_misc.p, 0, 64, s));
@@ -2055,7 +2056,8 @@ int sky_view_render(void* p, const SkyCamera* cam, const SkyViewSettings* vs, fl
   launch_viewer_ranges(I ? (const uint32_t*)c->v_tkeys_s.p : nullptr, I, tiles,
                        (uint32_t*)c->v_offsets.p, s);
   launch_viewer_raster(vp, (const float4*)c->v_splats.p, (const uint32_t*)c->v_offsets.p,
-                       I ? (const uint32_t*)c->v_gidx_s.p : nullptr, (float4*)c->v_rgba.p, s);
+                       I ? (const uint32_t*)c->v_gidx_s.p : nullptr, (float4*)c->v_rgba.p,
+                       rgba8 ? (uchar4*)c->v_rgba8.p : nullptr, s);
   c->launches += 2;
   CK(cudaGetLastError());
   uint32_t err = 0;
@@ -2064,20 +2066,8 @@ int sky_view_render(void* p, const SkyCamera* cam, const SkyViewSettings* vs, fl
   if (err & SKY_DEVERR_SORT_TIMEOUT) return fail(SKY_ERR_TIMEOUT, "radix sort look-back wait gave up");
   c->view_w = cam->width;
   c->view_h = cam->height;
-  if (rgba || rgba8) {
-    std::vector<float> tmp;
-    float* dst = rgba;
-    if (!dst) {
-      tmp.resize(px * 4);
-      dst = tmp.data();
-    }
-    CK(cudaMemcpy(dst, c->v_rgba.p, px * 16, cudaMemcpyDeviceToHost));
-    if (rgba8)
-      for (uint64_t i = 0; i < px * 4; ++i) {
-        const float v = std::min(std::max(dst[i], 0.0f), 1.0f);
-        rgba8[i] = (uint8_t)std::lround(v * 255.0f);
-      }
-  }
+  if (rgba) CK(cudaMemcpy(rgba, c->v_rgba.p, px * 16, cudaMemcpyDeviceToHost));
+  if (rgba8) CK(cudaMemcpy(rgba8, c->v_rgba8.p, px * 4, cudaMemcpyDeviceToHost));
   return SKY_OK;
 }
 

@@ -256,7 +256,7 @@ struct __align__(16) SplatPair {
 __global__ void __launch_bounds__(kViewTile* kViewTile, 5)
 k_viewer_raster(ViewerParams vp, const float4* __restrict__ splats,
                 const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ gidx,
-                float4* __restrict__ rgba) {
+                float4* __restrict__ rgba, uchar4* __restrict__ rgba8) {
   constexpr int NT = kViewTile * kViewTile;
   static_assert(kViewTile == 16 && kViewBatch == NT, "16-bit masks; one staged splat per thread");
   __shared__ float4 s_sp[kViewBatch][2];   // mean, conic a, b | conic c, opacity, red, green
@@ -353,7 +353,13 @@ k_viewer_raster(ViewerParams vp, const float4* __restrict__ splats,
       }
     }
   }
-  if (inside) rgba[(size_t)y * vp.width + x] = make_float4(C0, C1, C2, A);
+  if (inside) {
+    const size_t p = (size_t)y * vp.width + x;
+    rgba[p] = make_float4(C0, C1, C2, A);
+    // round(clamp(v, 0, 1) * 255), halves away from zero
+    auto u8 = [](float v) { return (unsigned char)lroundf(clampf_(v, 0.0f, 1.0f) * 255.0f); };
+    if (rgba8) rgba8[p] = make_uchar4(u8(C0), u8(C1), u8(C2), u8(A));
+  }
 }
 
 uint32_t blocks(uint32_t n, uint32_t t) { return (n + t - 1) / t; }
@@ -386,10 +392,10 @@ void launch_viewer_ranges(const uint32_t* tile_keys, uint32_t total, uint32_t ti
 }
 
 void launch_viewer_raster(const ViewerParams& vp, const float4* splats, const uint32_t* offsets,
-                          const uint32_t* gidx, float4* rgba, cudaStream_t s) {
+                          const uint32_t* gidx, float4* rgba, uchar4* rgba8, cudaStream_t s) {
   const uint32_t tiles = vp.tiles_x * vp.tiles_y;
   if (tiles)
-    k_viewer_raster<<<tiles, kViewTile * kViewTile, 0, s>>>(vp, splats, offsets, gidx, rgba);
+    k_viewer_raster<<<tiles, kViewTile * kViewTile, 0, s>>>(vp, splats, offsets, gidx, rgba, rgba8);
 }
 
 }  // namespace sky

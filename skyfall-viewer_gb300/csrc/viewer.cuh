@@ -37,8 +37,9 @@ void launch_viewer_emit(const ViewerParams& vp, const uint32_t* order, const uin
 // offsets[t] = first intersection of tile t (lower bound), offsets[T] = total.
 void launch_viewer_ranges(const uint32_t* tile_keys, uint32_t total, uint32_t tiles,
                           uint32_t* offsets, cudaStream_t s);
-// Back-to-front "over" blending of every splat whose quad covers the pixel.
+// Back-to-front "over" blending of every splat whose quad covers the pixel;
+// rgba8 (may be null) also receives the image as bytes.
 void launch_viewer_raster(const ViewerParams& vp, const float4* splats, const uint32_t* offsets,
-                          const uint32_t* gidx, float4* rgba, cudaStream_t s);
+                          const uint32_t* gidx, float4* rgba, uchar4* rgba8, cudaStream_t s);
 
 }  // namespace sky
