@@ -843,7 +843,7 @@ struct BoolC {
 // evaluates and composites and the list entries its warps walk; the
 // arithmetic and every result are those of the plain variant.
 template <int TS, int FB, bool CNT = false>
-__global__ void __launch_bounds__(TS* TS, TS == 16 ? 6 : 1) k_forward(DevBuffers b) {
+__global__ void __launch_bounds__(TS* TS, TS == 16 ? 6 : 1) k_forward(DevBuffers b, uint32_t first_tile) {
   static_assert(FB <= 256, "list entries are bytes");
   constexpr int NT = TS * TS;
   constexpr int NW = NT / 32;
@@ -855,7 +855,7 @@ __global__ void __launch_bounds__(TS* TS, TS == 16 ? 6 : 1) k_forward(DevBuffers
   __shared__ FwdPair s_pair[NW][CH / 2];
   __shared__ float4 s_tgt[NT];  // this thread's target pixel, copied in during the loop
   const StepParams& sp = *b.sp;
-  const uint32_t tile = blockIdx.x;
+  const uint32_t tile = first_tile + blockIdx.x;
   if (tile >= sp.num_tiles) return;
   if (capacity_failed(b.status)) return;
   const int v = find_view(sp, tile);
@@ -2719,27 +2719,33 @@ void launch_flatten_fill(const DevBuffers& b, uint32_t total, cudaStream_t s) {
 }
 
 template <int TS>
-void launch_forward_ts(const DevBuffers& b, uint32_t max_tiles, uint32_t fb, bool count,
+void launch_forward_ts(const DevBuffers& b, uint32_t first, uint32_t tiles, uint32_t fb, bool count,
                        cudaStream_t s) {
   if (TS == 16 && count && (fb == 0 || fb == (uint32_t)kFwdBatch)) {
-    k_forward<TS, kFwdBatch, true><<<max_tiles, TS * TS, 0, s>>>(b);
+    k_forward<TS, kFwdBatch, true><<<tiles, TS * TS, 0, s>>>(b, first);
     return;
   }
   switch (fb) {
-    case 64: k_forward<TS, 64><<<max_tiles, TS * TS, 0, s>>>(b); break;
-    case 128: k_forward<TS, 128><<<max_tiles, TS * TS, 0, s>>>(b); break;
-    default: k_forward<TS, kFwdBatch><<<max_tiles, TS * TS, 0, s>>>(b); break;
+    case 64: k_forward<TS, 64><<<tiles, TS * TS, 0, s>>>(b, first); break;
+    case 128: k_forward<TS, 128><<<tiles, TS * TS, 0, s>>>(b, first); break;
+    default: k_forward<TS, kFwdBatch><<<tiles, TS * TS, 0, s>>>(b, first); break;
+  }
+}
+
+void launch_forward_tiles(const DevBuffers& b, uint32_t first, uint32_t tiles, uint32_t ts, uint32_t fb,
+                          bool count, cudaStream_t s) {
+  if (tiles == 0) return;
+  switch (ts) {
+    case 8: launch_forward_ts<8>(b, first, tiles, fb, false, s); break;
+    case 32: launch_forward_ts<32>(b, first, tiles, fb, false, s); break;
+    default: launch_forward_ts<16>(b, first, tiles, fb, count, s); break;
   }
 }
 
 void launch_forward(const DevBuffers& b, uint32_t max_tiles, uint32_t ts, uint32_t fb, bool ssim,
                     uint32_t views, uint32_t max_view_pixels, bool count, cudaStream_t s) {
   if (max_tiles == 0) return;
-  switch (ts) {
-    case 8: launch_forward_ts<8>(b, max_tiles, fb, false, s); break;
-    case 32: launch_forward_ts<32>(b, max_tiles, fb, false, s); break;
-    default: launch_forward_ts<16>(b, max_tiles, fb, count, s); break;
-  }
+  launch_forward_tiles(b, 0, max_tiles, ts, fb, count, s);
   if (ssim) {
     dim3 grid((max_view_pixels + kSsimW * kSsimH - 1) / (kSsimW * kSsimH), views);
     k_ssim<<<grid, 256, 0, s>>>(b);

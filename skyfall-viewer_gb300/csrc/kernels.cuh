@@ -24,6 +24,9 @@ void launch_flatten_fill(const DevBuffers& b, uint32_t total, cudaStream_t s);
 constexpr uint32_t kBwdBatch16 = 64;  // default backward depth for 16x16 tiles
 // count: the pair-counting variants (16x16 tiles at the default depths
 // only; other shapes launch the plain kernels and count nothing).
+// The forward of tiles [first, first + tiles) alone (no SSIM term).
+void launch_forward_tiles(const DevBuffers& b, uint32_t first, uint32_t tiles, uint32_t ts, uint32_t fb,
+                          bool count, cudaStream_t s);
 void launch_forward(const DevBuffers& b, uint32_t max_tiles, uint32_t ts, uint32_t fb, bool ssim,
                     uint32_t views, uint32_t max_view_pixels, bool count, cudaStream_t s);
 // Doubles of b.loss_partials for a step of `tiles` tiles.
