@@ -1567,14 +1567,35 @@ int sky_knn_init(void* p, float scene_extent, float* density_out) {
   const uint32_t n = c->n;
   cudaStream_t s = c->stream;
   const float extent = scene_extent > 0.0f ? scene_extent : c->scene_extent;
-  TempBuf bounds(c), keys(c), ksorted(c), order(c), cstart(c), logs(c), dens(c), smem(c), pos(c);
-  TRY(dev_alloc(c, bounds.b, 64));
+  // one allocation for the call's scratch (an allocation and its release cost
+  // about 70 us each): the bounds, then what depends on n, then the cells
+  constexpr uint32_t kMaxCells = 1u << 22;
+  const size_t words = (((size_t)n * 4) + 255) & ~(size_t)255;
+  const size_t sort_bytes = (sort_scratch_bytes(n) + 255) & ~(size_t)255;
+  const uint32_t max_cells = (uint32_t)std::min<uint64_t>(kMaxCells, 4ull * n + 4096);
+  TempBuf mem(c);
+  TRY(dev_alloc(c, mem.b, 256 + 5 * words + 4 * words + sort_bytes + ((size_t)max_cells + 1) * 4));
+  char* at = (char*)mem.b.p;
+  auto take = [&](size_t bytes) {
+    char* r = at;
+    at += bytes;
+    return r;
+  };
+  uint32_t* const bounds = (uint32_t*)take(256);
+  uint32_t* const keys = (uint32_t*)take(words);
+  uint32_t* const ksorted = (uint32_t*)take(words);
+  uint32_t* const order = (uint32_t*)take(words);
+  float* const logs = (float*)take(words);
+  float* const dens = (float*)take(words);
+  float4* const pos = (float4*)take(4 * words);
+  char* const sort_mem = take(sort_bytes);
+  uint32_t* cstart = (uint32_t*)take(0);
   uint32_t init[6];
   for (int k = 0; k < 6; ++k) init[k] = knn_bounds_init(k);
-  CK(cudaMemcpyAsync(bounds.b.p, init, sizeof(init), cudaMemcpyHostToDevice, s));
-  launch_knn_bounds((const float*)c->params.p, c->stride, n, bounds.as<uint32_t>(), s);
+  CK(cudaMemcpyAsync(bounds, init, sizeof(init), cudaMemcpyHostToDevice, s));
+  launch_knn_bounds((const float*)c->params.p, c->stride, n, bounds, s);
   uint32_t bw[6];
-  CK(cudaMemcpyAsync(bw, bounds.b.p, sizeof(bw), cudaMemcpyDeviceToHost, s));
+  CK(cudaMemcpyAsync(bw, bounds, sizeof(bw), cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));
   // grid: about two points per cell over the bounding box, at most 2^22
   // cells and 1024 per axis
@@ -1607,32 +1628,29 @@ int sky_knn_init(void* p, float scene_extent, float* density_out) {
     h *= 1.25;
   }
   g.h = (float)h;
-  TRY(dev_alloc(c, keys.b, (size_t)n * 4));
-  TRY(dev_alloc(c, ksorted.b, (size_t)n * 4));
-  TRY(dev_alloc(c, order.b, (size_t)n * 4));
-  TRY(dev_alloc(c, cstart.b, ((size_t)g.cells + 1) * 4));
-  TRY(dev_alloc(c, logs.b, (size_t)n * 4));
-  TRY(dev_alloc(c, pos.b, (size_t)n * 16));
-  if (density_out) TRY(dev_alloc(c, dens.b, (size_t)n * 4));
-  TRY(dev_alloc(c, smem.b, sort_scratch_bytes(n)));
-  launch_knn_keys((const float*)c->params.p, c->stride, n, g, keys.as<uint32_t>(), s);
-  SortScratch sc = sort_scratch_carve(smem.b.p, n);
+  TempBuf more_cells(c);  // (a grid of more cells than the points make likely)
+  if (g.cells > max_cells) {
+    TRY(dev_alloc(c, more_cells.b, ((size_t)g.cells + 1) * 4));
+    cstart = more_cells.as<uint32_t>();
+  }
+  launch_knn_keys((const float*)c->params.p, c->stride, n, g, keys, s);
+  SortScratch sc = sort_scratch_carve(sort_mem, n);
   SortSegment seg{nullptr, n};
-  uint32_t* err = bounds.as<uint32_t>() + 8;
+  uint32_t* err = bounds + 8;
   CK(cudaMemsetAsync(err, 0, 4, s));
-  CK(sort_pairs_launch(keys.as<uint32_t>(), nullptr, ksorted.as<uint32_t>(), order.as<uint32_t>(), seg,
-                       n, std::max<uint32_t>(1, ceil_log2(g.cells)), sc, err, s));
-  launch_knn_cell_ranges(ksorted.as<uint32_t>(), n, g.cells, cstart.as<uint32_t>(), s);
-  launch_knn_query((const float*)c->params.p, c->stride, n, g, order.as<uint32_t>(),
-                   cstart.as<uint32_t>(), pos.as<float4>(), extent, dens.as<float>(), logs.as<float>(), s);
-  launch_knn_write((float*)c->params.p, c->stride, n, logs.as<float>(), s);
+  CK(sort_pairs_launch(keys, nullptr, ksorted, order, seg, n, std::max<uint32_t>(1, ceil_log2(g.cells)), sc,
+                       err, s));
+  launch_knn_cell_ranges(ksorted, n, g.cells, cstart, s);
+  launch_knn_query((const float*)c->params.p, c->stride, n, g, order, cstart, pos, extent,
+                   density_out ? dens : nullptr, logs, s);
+  launch_knn_write((float*)c->params.p, c->stride, n, logs, s);
   c->launches += 11;
   CK(cudaGetLastError());
   uint32_t e = 0;
   CK(cudaMemcpyAsync(&e, err, 4, cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));
   if (e & SKY_DEVERR_SORT_TIMEOUT) return fail(SKY_ERR_TIMEOUT, "radix sort look-back wait gave up");
-  if (density_out) CK(cudaMemcpy(density_out, dens.b.p, (size_t)n * 4, cudaMemcpyDeviceToHost));
+  if (density_out) CK(cudaMemcpy(density_out, dens, (size_t)n * 4, cudaMemcpyDeviceToHost));
   c->fwd_ready = false;
   c->scores_valid = false;
   return SKY_OK;
