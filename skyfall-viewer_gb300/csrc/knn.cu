@@ -208,13 +208,23 @@ k_knn_query(uint32_t n, KnnGrid g, const float4* __restrict__ pos, const uint32_
   log_sigma[self] = round_f16(sky_logf(fmax_(sig, 1e-6f)));
 }
 
+// One row of blocks per plane, four points per thread (the planes' padding up
+// to a multiple of four is the caller's stride): 236 bytes read and written per
+// point at 7.4 TB/s (part of them in L2), 62 -> 32 us for 500k against one
+// thread walking a point's 59 planes.
 __global__ void __launch_bounds__(256)
 k_knn_write(float* __restrict__ P, uint32_t stride, uint32_t n, const float* __restrict__ ls) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t i = 4u * (blockIdx.x * blockDim.x + threadIdx.x);
+  const uint32_t k = blockIdx.y;
   if (i >= n) return;
-  for (int k = 0; k < 59; ++k) {
-    float* v = P + (size_t)k * stride + i;
-    *v = (k >= 3 && k < 6) ? ls[i] : round_f16(*v);
+  float* v = P + (size_t)k * stride + i;
+  const bool scale = k >= 3u && k < 6u;
+  if (i + 4u <= n) {
+    float4 x = *reinterpret_cast<const float4*>(scale ? ls + i : v);
+    if (!scale) x = make_float4(round_f16(x.x), round_f16(x.y), round_f16(x.z), round_f16(x.w));
+    *reinterpret_cast<float4*>(v) = x;
+  } else {
+    for (uint32_t j = 0; i + j < n; ++j) v[j] = scale ? ls[i + j] : round_f16(v[j]);
   }
 }
 
@@ -256,7 +266,7 @@ void launch_knn_query(const float* params, uint32_t stride, uint32_t n, const Kn
 
 void launch_knn_write(float* params, uint32_t stride, uint32_t n, const float* log_sigma,
                       cudaStream_t s) {
-  if (n) k_knn_write<<<blocks(n), 256, 0, s>>>(params, stride, n, log_sigma);
+  if (n) k_knn_write<<<dim3((n + 1023) / 1024, 59), 256, 0, s>>>(params, stride, n, log_sigma);
 }
 
 }  // namespace sky
