@@ -12,6 +12,7 @@ constexpr uint32_t kFlagPrefix = 2u << 30;
 constexpr uint32_t kValueMask = (1u << 30) - 1u;
 constexpr uint32_t kSpinLimit = 1u << 20;
 constexpr int kWarps = kSortThreads / 32;
+constexpr int kLookBack = 2;
 
 __device__ __forceinline__ uint32_t ld_relaxed(const uint32_t* p) {
   uint32_t v;
@@ -242,9 +243,9 @@ k_onesweep(const uint32_t* keys_src, const uint32_t* vals_src, uint32_t* keys_ds
   // per digit bit, four where the upper ones do not vary (the item sorts'
   // depths).  match.any serialises over the distinct values of a round, about
   // 30 of 32 random bytes: 16.7M random keys 156 -> 136 us per pass; emission
-  // keys, in runs of equal digits, 125 -> 124.  Three blocks per multiprocessor
-  // (80 registers): four at 64 registers take 145 us, and look-back over eight
-  // predecessors per round trip 191 (115 registers).
+  // keys, in runs of equal digits, 125 -> 124.  Bound by the half-rate ALU pipe
+  // that the ballots' selects run on (73 % busy without the look-back); three
+  // blocks per multiprocessor (80 registers): four at 64 take 145 us.
   uint32_t rank[kSortItems / 2];  // two 16-bit ranks within the warp's digit per word
   auto rank_keys = [&](auto bits) {
 #pragma unroll
@@ -301,25 +302,39 @@ k_onesweep(const uint32_t* keys_src, const uint32_t* vals_src, uint32_t* keys_ds
   }
   if (lane == 31) s_scan[warp] = x;
 
-  // Decoupled look-back for this digit.
+  // Decoupled look-back for this digit, kLookBack predecessors per round trip:
+  // their words are loaded together and added in order up to the first
+  // inclusive prefix, or to the first that is not there yet, which is polled
+  // (one word: 134.5 us per pass of 16.7M random pairs, two: 131, four: 140,
+  // eight: 154 -- the words of 256 digits cost more than the round trips).
   uint32_t excl = 0;
   if (tile > 0) {
-    int64_t j = (int64_t)tile - 1;
+    int j = (int)tile - 1;
     uint32_t spins = 0;
-    while (j >= 0) {
-      uint32_t v = ld_relaxed(&lb[(uint64_t)j * kRadix + d]);
-      uint32_t flag = v & ~kValueMask;
-      if (flag == 0u) {
+    bool done = false;
+    while (!done && j >= 0) {
+      uint32_t v[kLookBack];
+#pragma unroll
+      for (int w = 0; w < kLookBack; ++w)
+        v[w] = j >= w ? ld_relaxed(&lb[(uint64_t)(uint32_t)(j - w) * kRadix + d]) : kFlagPrefix;
+      bool wait = false;
+#pragma unroll
+      for (int w = 0; w < kLookBack; ++w) {
+        const uint32_t flag = v[w] & ~kValueMask;
+        wait = wait || flag == 0u;
+        if (!done && !wait) {
+          excl += v[w] & kValueMask;
+          done = flag == kFlagPrefix;
+          --j;
+        }
+      }
+      if (wait && !done) {
         if (++spins > spin_limit) {
           atomicOr(err, SKY_DEVERR_SORT_TIMEOUT);
           break;
         }
         if (spins > 16) __nanosleep(64);
-        continue;
       }
-      excl += v & kValueMask;
-      if (flag == kFlagPrefix) break;
-      --j;
     }
     st_relaxed(&lb[(uint64_t)tile * kRadix + d], kFlagPrefix | (excl + run));
   }
