@@ -21,7 +21,8 @@ void launch_flatten_fill(const DevBuffers& b, uint32_t total, cudaStream_t s);
 // Splat-batch depths of the rasterizers: the forward stages fb splats per
 // batch (64, 128 or 256), the 16x16-tile exact backward bb (32, 64 or 128);
 // other values select the defaults.  Results do not depend on them.
-constexpr uint32_t kBwdBatch16 = 64;  // default backward depth for 16x16 tiles
+// Default backward depth for 16x16 tiles (few tiles: 128, k_backward_exact2).
+constexpr uint32_t kBwdBatch16 = 64;
 // count: the pair-counting variants (16x16 tiles at the default depths
 // only; other shapes launch the plain kernels and count nothing).
 // The forward of tiles [first, first + tiles) alone (no SSIM term).
