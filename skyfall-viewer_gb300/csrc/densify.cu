@@ -9,6 +9,7 @@
 // counter_uniform: draw r of Gaussian i at iteration t, so the results are
 // reproducible and independent of launch order.  The reference draws from
 // Math.random() in index order; the distributions are the same.
+#include "chain.cuh"
 #include "densify.cuh"
 #include "sky_math.cuh"
 
@@ -24,6 +25,7 @@ constexpr uint32_t kFull = 0xFFFFFFFFu;
 __global__ void __launch_bounds__(256)
 k_metric_partials(DevBuffers b, float* __restrict__ pmin, float* __restrict__ pmax,
                   double* __restrict__ psum) {
+  chain_wait();
   __shared__ float smin[8], smax[8];
   __shared__ double ssum[8];
   const ViewInfo& vi = b.sp->views[blockIdx.y];
@@ -70,6 +72,7 @@ k_metric_partials(DevBuffers b, float* __restrict__ pmin, float* __restrict__ pm
 __global__ void __launch_bounds__(32)
 k_metric_final(DevBuffers b, const float* __restrict__ pmin, const float* __restrict__ pmax,
                const double* __restrict__ psum, uint32_t nblocks, MetricStats* __restrict__ stats) {
+  chain_wait();
   const ViewInfo& vi = b.sp->views[blockIdx.x];
   const uint32_t npx = vi.width * vi.height;
   const size_t base = (size_t)blockIdx.x * nblocks;
@@ -100,6 +103,7 @@ k_metric_final(DevBuffers b, const float* __restrict__ pmin, const float* __rest
 __global__ void k_metric_combine(const uint32_t* __restrict__ counts, uint32_t n, uint32_t views,
                                  const MetricStats* __restrict__ st,
                                  uint32_t* __restrict__ importance, float* __restrict__ pruning) {
+  chain_wait();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   uint32_t imp = importance[i];
@@ -360,13 +364,13 @@ uint32_t blocks_for(uint32_t n, uint32_t threads) { return (n + threads - 1) / t
 
 void launch_metric_stats(const DevBuffers& b, uint32_t views, float* pmin, float* pmax, double* psum,
                          uint32_t nblocks, MetricStats* out, cudaStream_t s) {
-  k_metric_partials<<<dim3(nblocks, views), 256, 0, s>>>(b, pmin, pmax, psum);
-  k_metric_final<<<views, 32, 0, s>>>(b, pmin, pmax, psum, nblocks, out);
+  chain(k_metric_partials, dim3(nblocks, views), 256, 0, s, b, pmin, pmax, psum);
+  chain(k_metric_final, views, 32, 0, s, b, pmin, pmax, psum, nblocks, out);
 }
 
 void launch_metric_combine(const uint32_t* counts, uint32_t n, uint32_t views, const MetricStats* st,
                            uint32_t* importance, float* pruning, cudaStream_t s) {
-  if (n) k_metric_combine<<<blocks_for(n, 256), 256, 0, s>>>(counts, n, views, st, importance, pruning);
+  if (n) chain(k_metric_combine, blocks_for(n, 256), 256, 0, s, counts, n, views, st, importance, pruning);
 }
 
 void launch_densify_decide(const float* P, uint32_t stride, uint32_t n, const float4* accum,

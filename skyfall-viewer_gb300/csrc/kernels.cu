@@ -4,6 +4,7 @@
 // Adam.  Sort lives in sort.cu.  See kernels.cuh for the launch interface.
 #include "densify.cuh"
 #include "kernels.cuh"
+#include "chain.cuh"
 #include "project.cuh"
 
 #include <atomic>
@@ -363,6 +364,7 @@ SKY_DEV bool scan_skipped(const DevBuffers& b) { return b.status && capacity_fai
 // (all of a thread's loads are issued before the first is used: at 16k items
 // a loop of one load and one add took 10 us for four blocks)
 __global__ void __launch_bounds__(kScanThreads) k_scan_reduce(DevBuffers b, uint32_t n_items) {
+  chain_wait();
   __shared__ uint32_t s_warp[kScanThreads / 32];
   if (scan_skipped(b)) return;
   const uint32_t base = blockIdx.x * kScanTile + 4u * threadIdx.x;
@@ -382,6 +384,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_reduce(DevBuffers b, uint
 }
 
 __global__ void __launch_bounds__(1024) k_scan_blocks(DevBuffers b, uint32_t nblocks) {
+  chain_wait();
   __shared__ uint32_t s_warp[32];
   if (scan_skipped(b)) return;
   uint32_t carry = 0;
@@ -403,6 +406,7 @@ __global__ void __launch_bounds__(1024) k_scan_blocks(DevBuffers b, uint32_t nbl
 constexpr uint32_t kScanOwnPrefix = 4096;
 __global__ void __launch_bounds__(kScanThreads) k_scan_final(DevBuffers b, uint32_t n_items, bool own_prefix,
                                                              bool bounds) {
+  chain_wait();
   __shared__ uint32_t s_warp[kScanThreads / 32];
   if (scan_skipped(b)) return;
   const uint32_t base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
@@ -525,6 +529,7 @@ __global__ void k_group_bounds(DevBuffers b) {
 // contiguous range [end - count, end) of the emission order.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256, 6) k_emit(DevBuffers b) {
+  chain_wait();
   const StepParams& sp = *b.sp;
   const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t v = blockIdx.y;
@@ -614,6 +619,7 @@ __global__ void __launch_bounds__(256, 6) k_emit(DevBuffers b) {
 // last tile (the next group writes the same value there, the start of its
 // first; the last group's is the final sentinel).
 __global__ void __launch_bounds__(256) k_ranges(DevBuffers b) {
+  chain_wait();
   __shared__ uint32_t s_gb[kMaxGroups][2];
   __shared__ uint32_t s_gt[kMaxGroups][2];
   const StepParams& sp = *b.sp;
@@ -844,6 +850,7 @@ struct BoolC {
 // arithmetic and every result are those of the plain variant.
 template <int TS, int FB, bool CNT = false>
 __global__ void __launch_bounds__(TS* TS, TS == 16 ? 6 : 1) k_forward(DevBuffers b, uint32_t first_tile) {
+  chain_wait();
   static_assert(FB <= 256, "list entries are bytes");
   constexpr int NT = TS * TS;
   constexpr int NW = NT / 32;
@@ -1057,6 +1064,7 @@ SKY_DEV float div25(float x) {
 constexpr int kSsimW = 64, kSsimH = 16;         // output tile
 constexpr int kSsimP = 72, kSsimR = kSsimH + 4;  // row pitch (68 used), rows
 __global__ void __launch_bounds__(256, 4) k_ssim(DevBuffers b) {
+  chain_wait();
   __shared__ __align__(16) float s_im[2][3][kSsimR][kSsimP];  // rendered, target
   __shared__ __align__(16) float s_out[3][kSsimH][kSsimW];
   const StepParams& sp = *b.sp;
@@ -1164,6 +1172,7 @@ __global__ void __launch_bounds__(256, 4) k_ssim(DevBuffers b) {
 constexpr int kLossThreads = 256, kLossAhead = 16;
 constexpr uint32_t kLossSlice = kLossThreads * kLossAhead;  // tiles
 __global__ void __launch_bounds__(kLossThreads) k_loss_final(DevBuffers b) {
+  chain_wait();
   __shared__ double s[kLossThreads / 32];
   __shared__ uint32_t s_last;
   const StepParams& sp = *b.sp;
@@ -1272,6 +1281,7 @@ SKY_DEV int scatter9_slot(uint32_t lane) {
 
 template <int TS>
 __global__ void __launch_bounds__(TS* TS) k_backward_exact(DevBuffers b) {
+  chain_wait();
   constexpr int NT = TS * TS;
   constexpr int NW = NT / 32;
   constexpr int kBwdBatch = NW <= 8 ? 64 : 16;
@@ -1634,6 +1644,7 @@ constexpr int kFewTileBlocks = 5;
 constexpr uint32_t kFewTiles = kFewTileBlocks * 152;  // 152 multiprocessors
 template <int BB, bool CNT = false, bool FEW = false>
 __global__ void __launch_bounds__(128, FEW ? kFewTileBlocks : 8) k_backward_exact2(DevBuffers b) {
+  chain_wait();
   constexpr int TS = 16, NT = 128, NW = 4, kBatch = BB;
   static_assert(BB <= NT, "one staged splat per thread and batch");
   __shared__ BwdSplat s_rec[kBatch];
@@ -1852,6 +1863,7 @@ constexpr int kRefBatch = 64;
 
 template <int TS>
 __global__ void __launch_bounds__(TS* TS) k_backward_ref(DevBuffers b) {
+  chain_wait();
   constexpr int NT = TS * TS;
   __shared__ float4 s_rec[kRefBatch * 3];
   __shared__ float s_dir[kRefBatch * 3];
@@ -2010,6 +2022,7 @@ template <int TS>
 __global__ void __launch_bounds__(TS* TS)
 k_metric_accum(DevBuffers b, const MetricStats* __restrict__ stats, float threshold,
                uint32_t* __restrict__ counts) {
+  chain_wait();
   constexpr int NT = TS * TS, NW = NT / 32, FB = NT < 256 ? NT : 256;
   __shared__ float4 s_rec[FB];   // mean, conic a, b
   __shared__ float s_c[FB];      // conic c
@@ -2329,6 +2342,7 @@ constexpr int kGeomThreads = 128;
 // flagged in b.reached are read; the others are zero (intersections beyond
 // every pixel's last contributor, about half of them, and all-zero sums).
 __global__ void __launch_bounds__(256) k_item_sums(DevBuffers b) {
+  chain_wait();
   const StepParams& sp = *b.sp;
   if (capacity_failed(b.status)) return;
   const size_t items = (size_t)sp.num_views * sp.n;
@@ -2394,6 +2408,7 @@ constexpr size_t geom_smem() {
 static_assert(sizeof(ViewInfo) % 4 == 0, "cameras are copied as 32-bit words");
 template <bool FEW>
 __global__ void __launch_bounds__(kGeomThreads, FEW ? 4 : 3) k_geom_adam(DevBuffers b) {
+  chain_wait();
   extern __shared__ float4 s_dyn[];
   float* const s_base = reinterpret_cast<float*>(s_dyn);
   constexpr int kShRows = FEW ? 48 : 96;
@@ -2661,6 +2676,7 @@ SKY_DEV void sh_grads(const DevBuffers& b, const StepParams& sp, uint32_t g,
 }
 
 __global__ void __launch_bounds__(kShAdamThreads, 4) k_sh_adam(DevBuffers b) {
+  chain_wait();
   const StepParams& sp = *b.sp;
   if (!sp.sh_update || capacity_failed(b.status)) return;
   const uint32_t work = (sp.n + 4 * kShAdamThreads - 1) / (4 * kShAdamThreads) * kShGroups;
@@ -2720,9 +2736,9 @@ int launch_scan(const DevBuffers& b, uint32_t n_items, bool step, cudaStream_t s
   const uint32_t nb = (n_items + kScanTile - 1) / kScanTile;
   if (nb == 0) return 0;
   const bool own_prefix = nb <= kScanOwnPrefix;
-  k_scan_reduce<<<nb, kScanThreads, 0, s>>>(b, n_items);
-  if (!own_prefix) k_scan_blocks<<<1, 1024, 0, s>>>(b, nb);
-  k_scan_final<<<nb, kScanThreads, 0, s>>>(b, n_items, own_prefix, step);
+  chain(k_scan_reduce, nb, kScanThreads, 0, s, b, n_items);
+  if (!own_prefix) chain(k_scan_blocks, 1, 1024, 0, s, b, nb);
+  chain(k_scan_final, nb, kScanThreads, 0, s, b, n_items, own_prefix, step);
   return own_prefix ? 2 : 3;
 }
 
@@ -2732,12 +2748,12 @@ void launch_group_bounds(const DevBuffers& b, cudaStream_t s) { k_group_bounds<<
 
 void launch_emit(const DevBuffers& b, uint32_t n, uint32_t views, cudaStream_t s) {
   dim3 grid((n + 255) / 256, views);
-  k_emit<<<grid, 256, 0, s>>>(b);
+  chain(k_emit, grid, 256, 0, s, b);
 }
 
 void launch_ranges(const DevBuffers& b, uint32_t icap, cudaStream_t s) {
   const uint32_t blocks = min((icap / 4 + 255) / 256 + 1, (uint32_t)sm_count() * 8);
-  k_ranges<<<blocks, 256, 0, s>>>(b);
+  chain(k_ranges, blocks, 256, 0, s, b);
 }
 
 // Zeroes the partials the last backward did not write (unflagged), for a
@@ -2766,13 +2782,13 @@ template <int TS>
 void launch_forward_ts(const DevBuffers& b, uint32_t first, uint32_t tiles, uint32_t fb, bool count,
                        cudaStream_t s) {
   if (TS == 16 && count && (fb == 0 || fb == (uint32_t)kFwdBatch)) {
-    k_forward<TS, kFwdBatch, true><<<tiles, TS * TS, 0, s>>>(b, first);
+    chain(k_forward<TS, kFwdBatch, true>, tiles, TS * TS, 0, s, b, first);
     return;
   }
   switch (fb) {
-    case 64: k_forward<TS, 64><<<tiles, TS * TS, 0, s>>>(b, first); break;
-    case 128: k_forward<TS, 128><<<tiles, TS * TS, 0, s>>>(b, first); break;
-    default: k_forward<TS, kFwdBatch><<<tiles, TS * TS, 0, s>>>(b, first); break;
+    case 64: chain(k_forward<TS, 64>, tiles, TS * TS, 0, s, b, first); break;
+    case 128: chain(k_forward<TS, 128>, tiles, TS * TS, 0, s, b, first); break;
+    default: chain(k_forward<TS, kFwdBatch>, tiles, TS * TS, 0, s, b, first); break;
   }
 }
 
@@ -2792,14 +2808,14 @@ void launch_forward(const DevBuffers& b, uint32_t max_tiles, uint32_t ts, uint32
   launch_forward_tiles(b, 0, max_tiles, ts, fb, count, s);
   if (ssim) {
     dim3 grid((max_view_pixels + kSsimW * kSsimH - 1) / (kSsimW * kSsimH), views);
-    k_ssim<<<grid, 256, 0, s>>>(b);
+    chain(k_ssim, grid, 256, 0, s, b);
   }
 }
 
 size_t loss_partial_count(uint64_t tiles) { return (size_t)(tiles + tiles / kLossSlice + 1); }
 
 void launch_loss_final(const DevBuffers& b, uint32_t max_tiles, cudaStream_t s) {
-  k_loss_final<<<std::max(1u, std::min((max_tiles + kLossSlice - 1) / kLossSlice, 64u)), kLossThreads, 0, s>>>(b);
+  chain(k_loss_final, std::max(1u, std::min((max_tiles + kLossSlice - 1) / kLossSlice, 64u)), kLossThreads, 0, s, b);
 }
 
 void launch_backward(const DevBuffers& b, uint32_t max_tiles, uint32_t ts, uint32_t bb, bool ref,
@@ -2807,24 +2823,24 @@ void launch_backward(const DevBuffers& b, uint32_t max_tiles, uint32_t ts, uint3
   if (max_tiles == 0) return;
   if (!ref) {
     switch (ts) {
-      case 8: k_backward_exact<8><<<max_tiles, 64, 0, s>>>(b); break;
-      case 32: k_backward_exact<32><<<max_tiles, 1024, 0, s>>>(b); break;
+      case 8: chain(k_backward_exact<8>, max_tiles, 64, 0, s, b); break;
+      case 32: chain(k_backward_exact<32>, max_tiles, 1024, 0, s, b); break;
       default: {
         const bool few = max_tiles <= kFewTiles;
         if (count && (bb == 0 || bb == kBwdBatch16)) {
-          k_backward_exact2<kBwdBatch16, true><<<max_tiles, 128, 0, s>>>(b);
+          chain(k_backward_exact2<kBwdBatch16, true>, max_tiles, 128, 0, s, b);
           break;
         }
         switch (bb) {
-          case 32: k_backward_exact2<32><<<max_tiles, 128, 0, s>>>(b); break;
-          case 64: k_backward_exact2<64><<<max_tiles, 128, 0, s>>>(b); break;
+          case 32: chain(k_backward_exact2<32>, max_tiles, 128, 0, s, b); break;
+          case 64: chain(k_backward_exact2<64>, max_tiles, 128, 0, s, b); break;
           case 128:
-            if (few) k_backward_exact2<128, false, true><<<max_tiles, 128, 0, s>>>(b);
-            else k_backward_exact2<128><<<max_tiles, 128, 0, s>>>(b);
+            if (few) chain(k_backward_exact2<128, false, true>, max_tiles, 128, 0, s, b);
+            else chain(k_backward_exact2<128>, max_tiles, 128, 0, s, b);
             break;
           default:
-            if (few) k_backward_exact2<128, false, true><<<max_tiles, 128, 0, s>>>(b);
-            else k_backward_exact2<kBwdBatch16><<<max_tiles, 128, 0, s>>>(b);
+            if (few) chain(k_backward_exact2<128, false, true>, max_tiles, 128, 0, s, b);
+            else chain(k_backward_exact2<kBwdBatch16>, max_tiles, 128, 0, s, b);
             break;
         }
         break;
@@ -2832,9 +2848,9 @@ void launch_backward(const DevBuffers& b, uint32_t max_tiles, uint32_t ts, uint3
     }
   } else {
     switch (ts) {
-      case 8: k_backward_ref<8><<<max_tiles, 64, 0, s>>>(b); break;
-      case 32: k_backward_ref<32><<<max_tiles, 1024, 0, s>>>(b); break;
-      default: k_backward_ref<16><<<max_tiles, 256, 0, s>>>(b); break;
+      case 8: chain(k_backward_ref<8>, max_tiles, 64, 0, s, b); break;
+      case 32: chain(k_backward_ref<32>, max_tiles, 1024, 0, s, b); break;
+      default: chain(k_backward_ref<16>, max_tiles, 256, 0, s, b); break;
     }
   }
 }
@@ -2843,9 +2859,9 @@ void launch_metric_accum(const DevBuffers& b, uint32_t tiles, uint32_t ts, const
                          float threshold, uint32_t* counts, cudaStream_t s) {
   if (tiles == 0) return;
   switch (ts) {
-    case 8: k_metric_accum<8><<<tiles, 64, 0, s>>>(b, st, threshold, counts); break;
-    case 32: k_metric_accum<32><<<tiles, 1024, 0, s>>>(b, st, threshold, counts); break;
-    default: k_metric_accum<16><<<tiles, 256, 0, s>>>(b, st, threshold, counts); break;
+    case 8: chain(k_metric_accum<8>, tiles, 64, 0, s, b, st, threshold, counts); break;
+    case 32: chain(k_metric_accum<32>, tiles, 1024, 0, s, b, st, threshold, counts); break;
+    default: chain(k_metric_accum<16>, tiles, 256, 0, s, b, st, threshold, counts); break;
   }
 }
 
@@ -2861,7 +2877,7 @@ void launch_geom_adam_as(const DevBuffers& b, uint32_t n, cudaStream_t s) {
                          (int)geom_smem<FEW>());
     smem_set[dev].store(true, std::memory_order_release);
   }
-  k_geom_adam<FEW><<<(n + kGeomThreads - 1) / kGeomThreads, kGeomThreads, geom_smem<FEW>(), s>>>(b);
+  chain(k_geom_adam<FEW>, (n + kGeomThreads - 1) / kGeomThreads, kGeomThreads, geom_smem<FEW>(), s, b);
 }
 
 int launch_geom_adam(const DevBuffers& b, uint32_t n, uint32_t views, bool train_exact, cudaStream_t s) {
@@ -2875,14 +2891,14 @@ int launch_geom_adam(const DevBuffers& b, uint32_t n, uint32_t views, bool train
   // is a few empty blocks)
   const uint64_t work = (uint64_t)((n + 4 * kShAdamThreads - 1) / (4 * kShAdamThreads)) * kShGroups;
   const uint32_t blocks = (uint32_t)std::min<uint64_t>(work, (uint64_t)sm_count() * 16);
-  k_sh_adam<<<blocks, kShAdamThreads, 0, s>>>(b);
+  chain(k_sh_adam, blocks, kShAdamThreads, 0, s, b);
   return 2;
 }
 
 void launch_item_sums(const DevBuffers& b, uint64_t items, cudaStream_t s) {
   if (items == 0) return;
   const uint64_t blocks = std::min<uint64_t>((items + 255) / 256, (uint64_t)sm_count() * 16);
-  k_item_sums<<<(uint32_t)blocks, 256, 0, s>>>(b);
+  chain(k_item_sums, (uint32_t)blocks, 256, 0, s, b);
 }
 
 }  // namespace sky

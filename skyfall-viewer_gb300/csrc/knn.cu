@@ -11,6 +11,7 @@
 // reorder them), so the result is bit-identical to it.
 #include <cstring>
 
+#include "chain.cuh"
 #include "knn.cuh"
 #include "sky_math.cuh"
 
@@ -69,6 +70,7 @@ SKY_DEV uint32_t cell_of(float v, float lo, float h, uint32_t dim) {
 __global__ void __launch_bounds__(256)
 k_knn_keys(const float* __restrict__ P, uint32_t stride, uint32_t n, KnnGrid g,
            uint32_t* __restrict__ keys) {
+  chain_wait();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const uint32_t cx = cell_of(pos16(P, stride, 0, i), g.lo[0], g.h, g.dims[0]);
@@ -79,6 +81,7 @@ k_knn_keys(const float* __restrict__ P, uint32_t stride, uint32_t n, KnnGrid g,
 
 __global__ void k_knn_cell_ranges(const uint32_t* __restrict__ keys, uint32_t n, uint32_t cells,
                                   uint32_t* __restrict__ start) {
+  chain_wait();
   const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c > cells) return;
   uint32_t lo = 0, hi = n;
@@ -94,6 +97,7 @@ __global__ void k_knn_cell_ranges(const uint32_t* __restrict__ keys, uint32_t n,
 __global__ void __launch_bounds__(256)
 k_knn_gather(const float* __restrict__ P, uint32_t stride, uint32_t n,
              const uint32_t* __restrict__ order, float4* __restrict__ pos) {
+  chain_wait();
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   const uint32_t i = order[k];
@@ -125,6 +129,7 @@ SKY_DEV void insert3(float d[3], float v) {  // insert_sorted (knn-init.wgsl:27-
 __global__ void __launch_bounds__(256)
 k_knn_query(uint32_t n, KnnGrid g, const float4* __restrict__ pos, const uint32_t* __restrict__ start,
             float extent, float* __restrict__ density, float* __restrict__ log_sigma) {
+  chain_wait();
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   const float4 p = pos[k];
@@ -214,6 +219,7 @@ k_knn_query(uint32_t n, KnnGrid g, const float4* __restrict__ pos, const uint32_
 // thread walking a point's 59 planes.
 __global__ void __launch_bounds__(256)
 k_knn_write(float* __restrict__ P, uint32_t stride, uint32_t n, const float* __restrict__ ls) {
+  chain_wait();
   const uint32_t i = 4u * (blockIdx.x * blockDim.x + threadIdx.x);
   const uint32_t k = blockIdx.y;
   if (i >= n) return;
@@ -248,25 +254,25 @@ void launch_knn_bounds(const float* params, uint32_t stride, uint32_t n, uint32_
 
 void launch_knn_keys(const float* params, uint32_t stride, uint32_t n, const KnnGrid& g,
                      uint32_t* keys, cudaStream_t s) {
-  if (n) k_knn_keys<<<blocks(n), 256, 0, s>>>(params, stride, n, g, keys);
+  if (n) chain(k_knn_keys, blocks(n), 256, 0, s, params, stride, n, g, keys);
 }
 
 void launch_knn_cell_ranges(const uint32_t* keys_sorted, uint32_t n, uint32_t cells,
                             uint32_t* cell_start, cudaStream_t s) {
-  k_knn_cell_ranges<<<blocks(cells + 1), 256, 0, s>>>(keys_sorted, n, cells, cell_start);
+  chain(k_knn_cell_ranges, blocks(cells + 1), 256, 0, s, keys_sorted, n, cells, cell_start);
 }
 
 void launch_knn_query(const float* params, uint32_t stride, uint32_t n, const KnnGrid& g,
                       const uint32_t* order, const uint32_t* cell_start, float4* pos, float extent,
                       float* density, float* log_sigma, cudaStream_t s) {
   if (!n) return;
-  k_knn_gather<<<blocks(n), 256, 0, s>>>(params, stride, n, order, pos);
-  k_knn_query<<<blocks(n), 256, 0, s>>>(n, g, pos, cell_start, extent, density, log_sigma);
+  chain(k_knn_gather, blocks(n), 256, 0, s, params, stride, n, order, pos);
+  chain(k_knn_query, blocks(n), 256, 0, s, n, g, pos, cell_start, extent, density, log_sigma);
 }
 
 void launch_knn_write(float* params, uint32_t stride, uint32_t n, const float* log_sigma,
                       cudaStream_t s) {
-  if (n) k_knn_write<<<dim3((n + 1023) / 1024, 59), 256, 0, s>>>(params, stride, n, log_sigma);
+  if (n) chain(k_knn_write, dim3((n + 1023) / 1024, 59), 256, 0, s, params, stride, n, log_sigma);
 }
 
 }  // namespace sky

@@ -1,5 +1,6 @@
 // Onesweep LSD radix sort (see sort.cuh).
 #include "sort.cuh"
+#include "chain.cuh"
 
 #include <algorithm>
 #include <atomic>
@@ -52,6 +53,7 @@ __global__ void __launch_bounds__(kSortThreads)
 k_sort_hist(const uint32_t* __restrict__ keys, SortSegment seg, int passes, int digit_lo,
             uint32_t key_bits, uint32_t* __restrict__ hist, uint32_t* __restrict__ lookback,
             uint32_t max_tiles) {
+  chain_wait();
   __shared__ uint32_t s_hist[kMaxPasses][kRadix];
   for (int i = threadIdx.x; i < kMaxPasses * kRadix; i += kSortThreads) (&s_hist[0][0])[i] = 0;
   uint32_t begin, n;
@@ -132,6 +134,7 @@ k_sort_hist(const uint32_t* __restrict__ keys, SortSegment seg, int passes, int 
 // byte of the integer depth), and for passes below digit_lo.
 __global__ void __launch_bounds__(kRadix)
 k_sort_scan(uint32_t* __restrict__ hist, uint32_t* __restrict__ varying, int digit_lo) {
+  chain_wait();
   __shared__ uint32_t s_warp[kRadix / 32], s_or[kRadix / 32], s_and[kRadix / 32];
   uint32_t* h = hist + blockIdx.x * kRadix;
   uint32_t v = h[threadIdx.x];
@@ -177,6 +180,7 @@ k_onesweep(const uint32_t* keys_src, const uint32_t* vals_src, uint32_t* keys_ds
            const uint32_t* __restrict__ hist, uint32_t* __restrict__ tile_counter,
            uint32_t* __restrict__ lookback, uint32_t max_tiles, uint32_t* __restrict__ err,
            uint32_t spin_limit, uint32_t withhold_tile0) {
+  chain_wait();
   __shared__ uint32_t s_keys[kSortTile];
   __shared__ uint32_t s_vals[kSortTile];
   __shared__ uint32_t s_warp_hist[kWarps][kRadix];
@@ -433,10 +437,19 @@ cudaError_t sort_pairs_launch(const uint32_t* keys_in, const uint32_t* vals_in,
   uint32_t tiles = (max_n + kSortTile - 1) / kSortTile;
   if (tiles == 0) tiles = 1;
   uint32_t hist_blocks = tiles < 1024u ? tiles : 1024u;
-  k_sort_hist<<<hist_blocks, kSortThreads, 0, stream>>>(keys_in, seg, passes, digit_lo, key_bits,
-                                                         sc.hist, sc.lookback, sc.max_tiles);
+  // A capture of the caller's keeps ordinary edges between the kernels: a graph
+  // with programmatic ones does not answer every query (the step's own graph
+  // is only launched).
+  bool programmatic = true;
+  if (!cleared) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &st) != cudaSuccess) cudaGetLastError();
+    programmatic = st == cudaStreamCaptureStatusNone;
+  }
+  chain_if(programmatic, k_sort_hist, hist_blocks, kSortThreads, 0, stream, keys_in, seg, passes, digit_lo,
+           key_bits, sc.hist, sc.lookback, sc.max_tiles);
   uint32_t* varying = sc.tile_counter + 8;  // cleared with the tile tickets above
-  k_sort_scan<<<passes, kRadix, 0, stream>>>(sc.hist, varying, digit_lo);
+  chain_if(programmatic, k_sort_scan, passes, kRadix, 0, stream, sc.hist, varying, digit_lo);
   // Host fault injection (SKY_FAULT=lookback:N): in the N-th fault-point sort
   // of the process, tile 0 of every digit pass withholds its look-back word
   // and the waits give up after 64 polls -- the timeout path, without a
@@ -445,12 +458,10 @@ cudaError_t sort_pairs_launch(const uint32_t* keys_in, const uint32_t* vals_in,
   const bool inject = fault_point && fault_lookback_next(stream);
   const uint32_t spin_limit = inject ? 64u : kSpinLimit;
   for (int p = digit_lo; p < passes; ++p)
-    k_onesweep<<<std::min<uint32_t>(tiles, (uint32_t)sm_count() * 4), kSortThreads, 0,
-                 stream>>>(keys_in, vals_in, keys_out, vals_out,
-                                                    sc.keys_tmp, sc.vals_tmp, seg, p, passes,
-                                                    digit_lo, varying, key_bits, sc.hist,
-                                                    sc.tile_counter, sc.lookback, sc.max_tiles, err,
-                                                    spin_limit, inject ? 1u : 0u);
+    chain_if(programmatic, k_onesweep, std::min<uint32_t>(tiles, (uint32_t)sm_count() * 4), kSortThreads, 0,
+             stream, keys_in, vals_in, keys_out, vals_out, sc.keys_tmp, sc.vals_tmp, seg, p, passes, digit_lo,
+             varying, key_bits, sc.hist, sc.tile_counter, sc.lookback, sc.max_tiles, err, spin_limit,
+             inject ? 1u : 0u);
   return cudaGetLastError();
 }
 

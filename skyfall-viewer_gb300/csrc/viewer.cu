@@ -11,6 +11,7 @@
 // tested at pixel centres in f32 with the top-left rule (left and top quad
 // edges inside); a hardware rasterizer snaps quad corners to its sub-pixel
 // grid, so pixels within that snap of a quad edge can differ from it.
+#include "chain.cuh"
 #include "sky_math.cuh"
 #include "viewer.cuh"
 
@@ -193,6 +194,7 @@ k_viewer_project(ViewerParams vp, const float* __restrict__ P, float4* __restric
 __global__ void k_viewer_gather_counts(const uint32_t* __restrict__ order,
                                        const uint32_t* __restrict__ counts, uint32_t n,
                                        uint32_t* __restrict__ out) {
+  chain_wait();
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k < n) out[k] = counts[order[k]];
 }
@@ -201,6 +203,7 @@ __global__ void __launch_bounds__(256)
 k_viewer_emit(ViewerParams vp, const uint32_t* __restrict__ order, const uint32_t* __restrict__ cum,
               const uint32_t* __restrict__ counts_sorted, const uint2* __restrict__ rects,
               uint32_t n, uint32_t* __restrict__ tile_keys, uint32_t* __restrict__ gidx) {
+  chain_wait();
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   const uint32_t c = counts_sorted[k];
@@ -219,6 +222,7 @@ k_viewer_emit(ViewerParams vp, const uint32_t* __restrict__ order, const uint32_
 
 __global__ void k_viewer_ranges(const uint32_t* __restrict__ keys, uint32_t total, uint32_t tiles,
                                 uint32_t* __restrict__ offsets) {
+  chain_wait();
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t > tiles) return;
   uint32_t lo = 0, hi = total;  // first index with key >= t
@@ -257,6 +261,7 @@ __global__ void __launch_bounds__(kViewTile* kViewTile, 5)
 k_viewer_raster(ViewerParams vp, const float4* __restrict__ splats,
                 const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ gidx,
                 float4* __restrict__ rgba, uchar4* __restrict__ rgba8) {
+  chain_wait();
   constexpr int NT = kViewTile * kViewTile;
   static_assert(kViewTile == 16 && kViewBatch == NT, "16-bit masks; one staged splat per thread");
   __shared__ float4 s_sp[kViewBatch][2];   // mean, conic a, b | conic c, opacity, red, green
@@ -375,27 +380,27 @@ void launch_viewer_project(const ViewerParams& vp, const float* params, float4* 
 
 void launch_viewer_gather_counts(const uint32_t* order, const uint32_t* counts, uint32_t n,
                                  uint32_t* counts_sorted, cudaStream_t s) {
-  if (n) k_viewer_gather_counts<<<blocks(n, 256), 256, 0, s>>>(order, counts, n, counts_sorted);
+  if (n) chain(k_viewer_gather_counts, blocks(n, 256), 256, 0, s, order, counts, n, counts_sorted);
 }
 
 void launch_viewer_emit(const ViewerParams& vp, const uint32_t* order, const uint32_t* cum,
                         const uint32_t* counts_sorted, const uint2* rects, uint32_t n,
                         uint32_t* tile_keys, uint32_t* gidx, cudaStream_t s) {
   if (n)
-    k_viewer_emit<<<blocks(n, 256), 256, 0, s>>>(vp, order, cum, counts_sorted, rects, n, tile_keys,
+    chain(k_viewer_emit, blocks(n, 256), 256, 0, s, vp, order, cum, counts_sorted, rects, n, tile_keys,
                                                  gidx);
 }
 
 void launch_viewer_ranges(const uint32_t* tile_keys, uint32_t total, uint32_t tiles,
                           uint32_t* offsets, cudaStream_t s) {
-  k_viewer_ranges<<<blocks(tiles + 1, 256), 256, 0, s>>>(tile_keys, total, tiles, offsets);
+  chain(k_viewer_ranges, blocks(tiles + 1, 256), 256, 0, s, tile_keys, total, tiles, offsets);
 }
 
 void launch_viewer_raster(const ViewerParams& vp, const float4* splats, const uint32_t* offsets,
                           const uint32_t* gidx, float4* rgba, uchar4* rgba8, cudaStream_t s) {
   const uint32_t tiles = vp.tiles_x * vp.tiles_y;
   if (tiles)
-    k_viewer_raster<<<tiles, kViewTile * kViewTile, 0, s>>>(vp, splats, offsets, gidx, rgba, rgba8);
+    chain(k_viewer_raster, tiles, kViewTile * kViewTile, 0, s, vp, splats, offsets, gidx, rgba, rgba8);
 }
 
 }  // namespace sky
