@@ -525,50 +525,45 @@ __global__ void k_group_bounds(DevBuffers b) {
 // One thread per item in item order, so every read is coalesced: the
 // item's tile count, its emission end (scattered into item order by the
 // scan), its depth field (the item key the preprocess wrote), its rectangle
-// and, with culled lists, its record.  Each thread writes its item's
-// contiguous range [end - count, end) of the emission order.
+// and, with culled lists, its record.  An item's keys fill the contiguous range
+// [end - count, end) of the emission order.  Written by the item's own thread,
+// key by key, each is a 4-byte piece of a sector of its own per store: the
+// warp's keys go to shared memory instead (where a warp has at most kEmitStage,
+// 12 per item) and from there to memory with neighbouring lanes on neighbouring
+// words.  16 views of 1M Gaussians at 1080p 467 -> 315 us, a render of 8 317 ->
+// 145, one view with full rectangles 45 -> 24; 256 staged keys and eight blocks
+// per multiprocessor: 312, 160, 25; two items per thread: 318, 136, 23, but 16k
+// Gaussians 4.8 -> 5.9.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256, 6) k_emit(DevBuffers b) {
-  chain_wait();
-  const StepParams& sp = *b.sp;
-  const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
-  const uint32_t v = blockIdx.y;
-  if (g >= sp.n || v >= sp.num_views) return;
-  if (capacity_failed(b.status)) return;  // item_end / cumsum are not to be trusted
-  const uint32_t item = v * sp.n + g;
-  // every load the item needs is issued before the first branch, so their
-  // latencies overlap (most items are emitted)
-  const uint32_t cnt = b.counts[item];  // the rectangle's area, or the culled count
-  const uint32_t end = b.perm ? b.item_end[item] : b.cumsum[item];
-  const uint32_t ikey = b.ikeys[item];
-  const uint2 rc = b.rects[item];
-  const uint4 spans = sp.tile_cull ? b.rowspans[item] : make_uint4(0u, 0u, 0u, 0u);
-  if (cnt == 0u) return;
-  if (end > sp.icap || cnt > end) {
-    atomicOr(&b.status->error, SKY_DEVERR_LISTS);
-    return;
-  }
-  const uint32_t dq = ikey & 0xFFFFu;  // depth16 (depth_key of the item's depth)
-  const uint32_t x0 = rc.x & 0xFFFFu, y0 = rc.x >> 16, x1 = rc.y & 0xFFFFu, y1 = rc.y >> 16;
+constexpr uint32_t kEmitStage = 384;  // keys a warp stages
+struct EmitItem {
+  uint32_t cnt, end, ikey;
+  uint2 rc;
+  uint4 spans;
+};
+
+// put(k, key): the key of the item's k-th tile.  Returns false if the item
+// lists other than cnt tiles (put is called for the first cnt of them).
+template <class Put>
+SKY_DEV bool emit_item(const DevBuffers& b, const StepParams& sp, uint32_t tile0, uint32_t tiles_x,
+                       uint32_t item, const EmitItem& d, Put put) {
+  const uint32_t cnt = d.cnt;
+  const uint32_t dq = d.ikey & 0xFFFFu;  // depth16 (depth_key of the item's depth)
+  const uint32_t x0 = d.rc.x & 0xFFFFu, y0 = d.rc.x >> 16, x1 = d.rc.y & 0xFFFFu, y1 = d.rc.y >> 16;
   const uint32_t area = (x1 <= x0 || y1 <= y0) ? 0u : (x1 - x0) * (y1 - y0);
-  uint32_t cur = end - cnt;
-  const ViewInfo& vi = sp.views[v];
+  uint32_t k = 0;
   // the keys of tiles [lo, lo + len) of tile row ty; false: the row holds
   // more tiles than the item's range has left (lists counted differently)
   auto emit_row = [&](uint32_t ty, uint32_t lo, uint32_t len) {
-    if (len > end - cur) return false;
-    for (uint32_t tx = lo; tx < lo + len; ++tx) {
-      const uint32_t kt = vi.key_tile_base + ty * vi.tiles_x + tx;
-      b.keys[cur] = (kt << 16) | dq;
-      b.rec_of[cur] = item;
-      ++cur;
-    }
+    if (len > cnt - k) return false;
+    uint32_t key = ((tile0 + ty * tiles_x + lo) << 16) | dq;
+    for (const uint32_t stop = k + len; k < stop; ++k, key += 1u << 16) put(k, key);
     return true;
   };
   bool ok = true;
   if (cnt == area) {
     for (uint32_t ty = y0; ty < y1; ++ty) emit_row(ty, x0, x1 - x0);
-    return;
+    return true;
   }
   // culled: the tiles the preprocess counted -- its row spans where it kept
   // them, else the same test on the same record values
@@ -576,7 +571,7 @@ __global__ void __launch_bounds__(256, 6) k_emit(DevBuffers b) {
     ok = false;
   } else if (y1 - y0 <= kSpanRows && x1 - x0 <= 255u) {
     for (uint32_t r = 0; ok && r < y1 - y0; ++r) {
-      const uint32_t wv = r < 2u ? spans.x : (r < 4u ? spans.y : (r < 6u ? spans.z : spans.w));
+      const uint32_t wv = r < 2u ? d.spans.x : (r < 4u ? d.spans.y : (r < 6u ? d.spans.z : d.spans.w));
       const uint32_t h = (wv >> (16u * (r & 1u))) & 0xFFFFu;
       ok = emit_row(y0 + r, x0 + (h & 0xFFu), h >> 8);
     }
@@ -592,8 +587,69 @@ __global__ void __launch_bounds__(256, 6) k_emit(DevBuffers b) {
       ok = emit_row(ty, lo, len);
     }
   }
-  // counted differently from the preprocess: corrupt lists
-  if (!ok || cur != end) atomicOr(&b.status->error, SKY_DEVERR_LISTS);
+  ok = ok && k == cnt;
+  for (; k < cnt; ++k) put(k, dq);  // (corrupt lists: nothing reads them)
+  return ok;
+}
+
+__global__ void __launch_bounds__(256, 6) k_emit(DevBuffers b) {
+  chain_wait();
+  __shared__ uint32_t s_key[8][kEmitStage];
+  __shared__ uint8_t s_own[8][kEmitStage];  // the lane whose item a staged key is
+  const StepParams& sp = *b.sp;
+  const uint32_t v = blockIdx.y;
+  if (v >= sp.num_views || capacity_failed(b.status)) return;  // item_end / cumsum are not to be trusted
+  const uint32_t tile0 = sp.views[v].key_tile_base, tiles_x = sp.views[v].tiles_x;
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x, item = v * sp.n + g;
+  // every load the item needs is issued before the first branch, so their
+  // latencies overlap (most items are emitted)
+  EmitItem d{};
+  if (g < sp.n) {
+    d.cnt = b.counts[item];  // the rectangle's area, or the culled count
+    d.end = b.perm ? b.item_end[item] : b.cumsum[item];
+    d.ikey = b.ikeys[item];
+    d.rc = b.rects[item];
+    if (sp.tile_cull) d.spans = b.rowspans[item];
+  }
+  bool ok = d.cnt == 0u || (d.end <= sp.icap && d.cnt <= d.end);
+  if (!ok) d.cnt = 0u;
+  const uint32_t cnt = d.cnt, first = d.end - cnt;
+  const uint32_t staged = min(cnt, kEmitStage + 1u);  // (the sum does not wrap)
+  uint32_t incl = staged;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(kFull, incl, o);
+    if (lane >= (uint32_t)o) incl += y;
+  }
+  const uint32_t total = __shfl_sync(kFull, incl, 31), excl = incl - staged;
+  if (total <= kEmitStage) {
+    uint32_t* const keys = s_key[warp];
+    uint8_t* const own = s_own[warp];
+    if (cnt != 0u)
+      ok = emit_item(b, sp, tile0, tiles_x, item, d, [&](uint32_t k, uint32_t key) {
+        keys[excl + k] = key;
+        own[excl + k] = (uint8_t)lane;
+      });
+    __syncwarp();
+    const uint32_t base = first - excl;  // of the item's staged keys (modulo 2^32)
+    for (uint32_t t = 0; t < total; t += 32) {
+      const uint32_t o = t + lane;
+      const uint32_t w = o < total ? own[o] : 0u;
+      const uint32_t dst = __shfl_sync(kFull, base, (int)w) + o;
+      if (o < total) {
+        b.keys[dst] = keys[o];
+        b.rec_of[dst] = item - lane + w;
+      }
+    }
+  } else if (cnt != 0u) {
+    ok = emit_item(b, sp, tile0, tiles_x, item, d, [&](uint32_t k, uint32_t key) {
+      b.keys[first + k] = key;
+      b.rec_of[first + k] = item;
+    });
+  }
+  // not what the preprocess counted: corrupt lists
+  if (!ok) atomicOr(&b.status->error, SKY_DEVERR_LISTS);
 }
 
 // ---------------------------------------------------------------------------
