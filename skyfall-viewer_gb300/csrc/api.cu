@@ -483,7 +483,16 @@ void drop_graph(Context* c) {
 // the link), and in chunks of at least 2048 tiles, two waves of the forward's
 // blocks.  8 views of 1M Gaussians at 1080p (331 MB): 5.32 ms in one launch
 // and one copy, 3.99 in 8 chunks on one stream, 3.85 on two streams in turn,
-// 3.72 in 16.
+// 3.72 in 16.  Only into page-locked memory: a 4K view into pageable memory
+// takes 77 ms in chunks and 7.4 in one copy.
+bool page_locked(const void* p) {
+  if (!p) return true;
+  cudaPointerAttributes a{};
+  if (cudaPointerGetAttributes(&a, p) == cudaSuccess) return a.type == cudaMemoryTypeHost;
+  cudaGetLastError();
+  return false;
+}
+
 std::vector<Chunk> render_chunks(const StepParams& sp, uint64_t bytes_per_px) {
   std::vector<Chunk> out;
   const uint64_t bytes = (uint64_t)sp.num_pixels * bytes_per_px;
@@ -700,7 +709,8 @@ int run_views(Context* c, const uint32_t* cams, uint32_t nv, Mode mode, SkyStepS
   cudaStream_t s = c->stream;
   uint64_t launches = 0, h2d = 0, d2h = 0;
   std::vector<Chunk> chunks;
-  if (out) chunks = render_chunks(sp, (out->rgba ? 16 : 0) + (out->alpha ? 4 : 0));
+  if (out && page_locked(out->rgba) && page_locked(out->alpha))
+    chunks = render_chunks(sp, (out->rgba ? 16 : 0) + (out->alpha ? 4 : 0));
   if (!chunks.empty() && !c->ready) {
     if (!c->copy_stream) CK(cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking));
     if (!c->chunk_stream) CK(cudaStreamCreateWithFlags(&c->chunk_stream, cudaStreamNonBlocking));
