@@ -350,7 +350,8 @@ int sky_set_target(void* ctx, uint32_t camera, const float* rgb, uint32_t width,
 
 /* ---- hot path --------------------------------------------------------------
  * sky_render: forward only for n cameras; rgba (4 f32) and alpha (1 f32) per
- * pixel, images concatenated in camera order (either pointer may be NULL).
+ * pixel, images concatenated in camera order (either pointer may be NULL;
+ * large images in page-locked memory leave while later tiles are rendered).
  * sky_forward + sky_backward: the forward/backward op pair; sky_forward also
  * evaluates the loss against the cameras' targets, sky_backward returns the
  * 59 gradient planes (summed over the forward's views) without an Adam step.
