@@ -12,6 +12,8 @@
 
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 namespace sky {
 
 // The first statement of every kernel that chain() launches: waits until the
@@ -19,7 +21,20 @@ namespace sky {
 // (nothing to wait for after a plain launch).  Every block runs it, also those
 // with no work: a kernel that completed before its predecessor would let its
 // own successor start too early.
-__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// p: every pointer parameter of the kernel.  Loads through a const __restrict__
+// parameter are invariant to the compiler, which may move them above a memory
+// clobber; passed through an empty volatile statement behind the wait, the
+// pointers, and with them the loads, cannot go before it.
+template <class... P>
+__device__ __forceinline__ void chain_wait(P&... p) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  auto behind = [](auto& q) {
+    unsigned long long a = reinterpret_cast<unsigned long long>(q);
+    asm volatile("" : "+l"(a)::"memory");
+    q = reinterpret_cast<std::remove_reference_t<decltype(q)>>(a);
+  };
+  (behind(p), ...);
+}
 
 // programmatic: false launches as <<<>>> does.
 template <class... P, class... A>

@@ -25,7 +25,7 @@ constexpr uint32_t kFull = 0xFFFFFFFFu;
 __global__ void __launch_bounds__(256)
 k_metric_partials(DevBuffers b, float* __restrict__ pmin, float* __restrict__ pmax,
                   double* __restrict__ psum) {
-  chain_wait();
+  chain_wait(pmin, pmax, psum);
   __shared__ float smin[8], smax[8];
   __shared__ double ssum[8];
   const ViewInfo& vi = b.sp->views[blockIdx.y];
@@ -72,7 +72,7 @@ k_metric_partials(DevBuffers b, float* __restrict__ pmin, float* __restrict__ pm
 __global__ void __launch_bounds__(32)
 k_metric_final(DevBuffers b, const float* __restrict__ pmin, const float* __restrict__ pmax,
                const double* __restrict__ psum, uint32_t nblocks, MetricStats* __restrict__ stats) {
-  chain_wait();
+  chain_wait(pmin, pmax, psum, stats);
   const ViewInfo& vi = b.sp->views[blockIdx.x];
   const uint32_t npx = vi.width * vi.height;
   const size_t base = (size_t)blockIdx.x * nblocks;
@@ -103,7 +103,7 @@ k_metric_final(DevBuffers b, const float* __restrict__ pmin, const float* __rest
 __global__ void k_metric_combine(const uint32_t* __restrict__ counts, uint32_t n, uint32_t views,
                                  const MetricStats* __restrict__ st,
                                  uint32_t* __restrict__ importance, float* __restrict__ pruning) {
-  chain_wait();
+  chain_wait(counts, st, importance, pruning);
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   uint32_t imp = importance[i];

@@ -2080,7 +2080,7 @@ template <int TS>
 __global__ void __launch_bounds__(TS* TS)
 k_metric_accum(DevBuffers b, const MetricStats* __restrict__ stats, float threshold,
                uint32_t* __restrict__ counts) {
-  chain_wait();
+  chain_wait(stats, counts);
   constexpr int NT = TS * TS, NW = NT / 32, FB = NT < 256 ? NT : 256;
   __shared__ float4 s_rec[FB];   // mean, conic a, b
   __shared__ float s_c[FB];      // conic c

@@ -70,7 +70,7 @@ SKY_DEV uint32_t cell_of(float v, float lo, float h, uint32_t dim) {
 __global__ void __launch_bounds__(256)
 k_knn_keys(const float* __restrict__ P, uint32_t stride, uint32_t n, KnnGrid g,
            uint32_t* __restrict__ keys) {
-  chain_wait();
+  chain_wait(P, keys);
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const uint32_t cx = cell_of(pos16(P, stride, 0, i), g.lo[0], g.h, g.dims[0]);
@@ -81,7 +81,7 @@ k_knn_keys(const float* __restrict__ P, uint32_t stride, uint32_t n, KnnGrid g,
 
 __global__ void k_knn_cell_ranges(const uint32_t* __restrict__ keys, uint32_t n, uint32_t cells,
                                   uint32_t* __restrict__ start) {
-  chain_wait();
+  chain_wait(keys, start);
   const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c > cells) return;
   uint32_t lo = 0, hi = n;
@@ -97,7 +97,7 @@ __global__ void k_knn_cell_ranges(const uint32_t* __restrict__ keys, uint32_t n,
 __global__ void __launch_bounds__(256)
 k_knn_gather(const float* __restrict__ P, uint32_t stride, uint32_t n,
              const uint32_t* __restrict__ order, float4* __restrict__ pos) {
-  chain_wait();
+  chain_wait(P, order, pos);
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   const uint32_t i = order[k];
@@ -129,7 +129,7 @@ SKY_DEV void insert3(float d[3], float v) {  // insert_sorted (knn-init.wgsl:27-
 __global__ void __launch_bounds__(256)
 k_knn_query(uint32_t n, KnnGrid g, const float4* __restrict__ pos, const uint32_t* __restrict__ start,
             float extent, float* __restrict__ density, float* __restrict__ log_sigma) {
-  chain_wait();
+  chain_wait(pos, start, density, log_sigma);
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   const float4 p = pos[k];
@@ -219,7 +219,7 @@ k_knn_query(uint32_t n, KnnGrid g, const float4* __restrict__ pos, const uint32_
 // thread walking a point's 59 planes.
 __global__ void __launch_bounds__(256)
 k_knn_write(float* __restrict__ P, uint32_t stride, uint32_t n, const float* __restrict__ ls) {
-  chain_wait();
+  chain_wait(P, ls);
   const uint32_t i = 4u * (blockIdx.x * blockDim.x + threadIdx.x);
   const uint32_t k = blockIdx.y;
   if (i >= n) return;

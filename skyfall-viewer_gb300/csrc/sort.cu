@@ -53,7 +53,7 @@ __global__ void __launch_bounds__(kSortThreads)
 k_sort_hist(const uint32_t* __restrict__ keys, SortSegment seg, int passes, int digit_lo,
             uint32_t key_bits, uint32_t* __restrict__ hist, uint32_t* __restrict__ lookback,
             uint32_t max_tiles) {
-  chain_wait();
+  chain_wait(keys, hist, lookback);
   __shared__ uint32_t s_hist[kMaxPasses][kRadix];
   for (int i = threadIdx.x; i < kMaxPasses * kRadix; i += kSortThreads) (&s_hist[0][0])[i] = 0;
   uint32_t begin, n;
@@ -134,7 +134,7 @@ k_sort_hist(const uint32_t* __restrict__ keys, SortSegment seg, int passes, int 
 // byte of the integer depth), and for passes below digit_lo.
 __global__ void __launch_bounds__(kRadix)
 k_sort_scan(uint32_t* __restrict__ hist, uint32_t* __restrict__ varying, int digit_lo) {
-  chain_wait();
+  chain_wait(hist, varying);
   __shared__ uint32_t s_warp[kRadix / 32], s_or[kRadix / 32], s_and[kRadix / 32];
   uint32_t* h = hist + blockIdx.x * kRadix;
   uint32_t v = h[threadIdx.x];
@@ -180,7 +180,7 @@ k_onesweep(const uint32_t* keys_src, const uint32_t* vals_src, uint32_t* keys_ds
            const uint32_t* __restrict__ hist, uint32_t* __restrict__ tile_counter,
            uint32_t* __restrict__ lookback, uint32_t max_tiles, uint32_t* __restrict__ err,
            uint32_t spin_limit, uint32_t withhold_tile0) {
-  chain_wait();
+  chain_wait(keys_src, vals_src, keys_dst_out, vals_dst_out, keys_tmp, vals_tmp, varying, hist, tile_counter, lookback, err);
   __shared__ uint32_t s_keys[kSortTile];
   __shared__ uint32_t s_vals[kSortTile];
   __shared__ uint32_t s_warp_hist[kWarps][kRadix];

@@ -194,7 +194,7 @@ k_viewer_project(ViewerParams vp, const float* __restrict__ P, float4* __restric
 __global__ void k_viewer_gather_counts(const uint32_t* __restrict__ order,
                                        const uint32_t* __restrict__ counts, uint32_t n,
                                        uint32_t* __restrict__ out) {
-  chain_wait();
+  chain_wait(order, counts, out);
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k < n) out[k] = counts[order[k]];
 }
@@ -208,7 +208,7 @@ __global__ void __launch_bounds__(256)
 k_viewer_emit(ViewerParams vp, const uint32_t* __restrict__ order, const uint32_t* __restrict__ cum,
               const uint32_t* __restrict__ counts_sorted, const uint2* __restrict__ rects,
               uint32_t n, uint32_t* __restrict__ tile_keys, uint32_t* __restrict__ gidx) {
-  chain_wait();
+  chain_wait(order, cum, counts_sorted, rects, tile_keys, gidx);
   __shared__ uint32_t s_key[8][kEmitStage];
   __shared__ uint8_t s_own[8][kEmitStage];  // the lane whose Gaussian a staged key is
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -252,7 +252,7 @@ k_viewer_emit(ViewerParams vp, const uint32_t* __restrict__ order, const uint32_
 
 __global__ void k_viewer_ranges(const uint32_t* __restrict__ keys, uint32_t total, uint32_t tiles,
                                 uint32_t* __restrict__ offsets) {
-  chain_wait();
+  chain_wait(keys, offsets);
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t > tiles) return;
   uint32_t lo = 0, hi = total;  // first index with key >= t
@@ -291,7 +291,7 @@ __global__ void __launch_bounds__(kViewTile* kViewTile, 5)
 k_viewer_raster(ViewerParams vp, const float4* __restrict__ splats,
                 const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ gidx,
                 float4* __restrict__ rgba, uchar4* __restrict__ rgba8) {
-  chain_wait();
+  chain_wait(splats, offsets, gidx, rgba, rgba8);
   constexpr int NT = kViewTile * kViewTile;
   static_assert(kViewTile == 16 && kViewBatch == NT, "16-bit masks; one staged splat per thread");
   __shared__ float4 s_sp[kViewBatch][2];   // mean, conic a, b | conic c, opacity, red, green
