@@ -402,9 +402,9 @@ int enqueue(Context* c, const Shape& sh, bool sizing_sync, bool capturing, const
     d2h += sizeof(DevStatus);
     CK(cudaMemcpyAsync(c->h_st, c->d_st.p, sizeof(DevStatus), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
-    // (the capacity bit is the group-bounds kernel's request to grow; after
-    // a sort that gave up the later kernels of the step do nothing and the
-    // count is not to be trusted: no growth)
+    // (the capacity bit is the scan's request to grow; after a sort that gave
+    // up the later kernels of the step do nothing and the count is not to be
+    // trusted: no growth)
     const uint32_t fatal = c->h_st->error & ~SKY_DEVERR_CAPACITY;
     if (fatal == 0u && c->h_st->total_isect > c->icap) {
       TRY(ensure_isect(c, c->h_st->total_isect));
@@ -804,6 +804,8 @@ int run_views(Context* c, const uint32_t* cams, uint32_t nv, Mode mode, SkyStepS
     return fail(SKY_ERR_STATE,
                 "intersection lists inconsistent: key emission disagreed with the preprocess's "
                 "tile counts, or the tile ranges met unsorted keys");
+  if (c->h_st->error & SKY_DEVERR_VIEWS)
+    return fail(SKY_ERR_CAPACITY, "pass launched for fewer views than its parameters name");
   if (c->h_st->error & SKY_DEVERR_CAPACITY)
     return fail(SKY_ERR_CAPACITY, "intersection capacity exceeded");
   c->sized = true;

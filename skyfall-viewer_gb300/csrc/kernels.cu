@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(kPrepThreads, 8) k_preprocess(DevBuffers b) {
     uint32_t dyn;
     asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn));
     if (sp.num_views * (uint32_t)sizeof(ViewInfo) > dyn) {  // launched for fewer views
-      if (threadIdx.x == 0) atomicOr(&b.status->error, SKY_DEVERR_CAPACITY);
+      if (threadIdx.x == 0) atomicOr(&b.status->error, SKY_DEVERR_VIEWS);
       return;
     }
     const uint32_t words = sp.num_views * (uint32_t)(sizeof(ViewInfo) / 4);
@@ -359,7 +359,9 @@ SKY_DEV uint32_t scan_count(const DevBuffers& b, uint32_t word, uint32_t i) {
 
 // A scan of a step (b.status set) after a sort that gave up does nothing:
 // the permutation may hold stale words, which must not be used as indices.
-SKY_DEV bool scan_skipped(const DevBuffers& b) { return b.status && capacity_failed(b.status); }
+SKY_DEV bool scan_skipped(const DevBuffers& b) {
+  return b.status && scan_without_input(*(volatile const uint32_t*)&b.status->error);
+}
 
 // (all of a thread's loads are issued before the first is used: at 16k items
 // a loop of one load and one add took 10 us for four blocks)

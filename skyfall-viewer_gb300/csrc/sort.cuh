@@ -30,6 +30,14 @@ constexpr uint32_t SKY_DEVERR_SORT_TIMEOUT = 2u;
 // different number of tiles than the preprocess counted for an item, or the
 // tile ranges met sorted keys out of order.  Later kernels of the step skip.
 constexpr uint32_t SKY_DEVERR_LISTS = 4u;
+// The step's parameters name more views than it was launched for.
+constexpr uint32_t SKY_DEVERR_VIEWS = 8u;
+
+// Whether an error before a step's scan leaves it nothing to scan.  The capacity
+// bit does not: the scan raises it itself, at its last item, when other blocks
+// of its grid may not have read the word yet, and a pass that grows its buffers
+// goes on with what those blocks write.
+__host__ __device__ inline bool scan_without_input(uint32_t error) { return (error & ~SKY_DEVERR_CAPACITY) != 0u; }
 
 // Cleared before every sort: the digit counts and, behind them, the tickets.
 constexpr size_t kSortClearBytes = (size_t)kMaxPasses * kRadix * 4 + 256;
