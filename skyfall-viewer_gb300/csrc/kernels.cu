@@ -1617,7 +1617,11 @@ SKY_DEV bool bwd_pixels(BwdPix2& p, const BwdSplat& q, int j, const int (&jmin)[
     if (!v0) r[0][0] = r[0][1] = r[0][2] = dd[0] = 0.0f;
     if (!v1) r[1][0] = r[1][1] = r[1][2] = dd[1] = 0.0f;
   }
-  const float dl[2] = {dd[0] * Tb.x, dd[1] * Tb.y};
+  float dl[2] = {dd[0] * Tb.x, dd[1] * Tb.y};
+  if constexpr (!FIN) {  // (nor does the clamp pass on more than a finite value times 0)
+    if (al.x == 0.0f) dl[0] = 0.0f;
+    if (al.y == 0.0f) dl[1] = 0.0f;
+  }
   const float g[2] = {dl[0] * al.x, dl[1] * al.y};
   const float gdy[2] = {g[0] * dy.x, g[1] * dy.y};
 #pragma unroll
