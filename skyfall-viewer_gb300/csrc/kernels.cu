@@ -1565,7 +1565,8 @@ struct __align__(16) BwdSplat {
 // which makes its terms 0 and leaves racc and T alone (T / 1 is T: the quotient
 // multiplies by the reciprocal of 1, which is exact) -- as long as the
 // residual, the colour and their products are finite (FIN, both below
-// kBwdFinite); otherwise its operands are cleared too.  With a branch per
+// kBwdFinite, the colours of the batches before too: racc); otherwise its
+// operands are cleared too.  With a branch per
 // pixel, lanes of both kinds run both sides of nearly every entry.
 constexpr float kBwdFinite = 1e18f;
 template <bool FIN, bool CNT>
@@ -1749,7 +1750,8 @@ __global__ void __launch_bounds__(128, FEW ? kFewTileBlocks : 8) k_backward_exac
         r[0][h] = rs.x; r[1][h] = rs.y; r[2][h] = rs.z;
       }
       racc[h] = __fmaf_rn(r[2][h], sp.bg[2], __fmaf_rn(r[1][h], sp.bg[1], r[0][h] * sp.bg[0]));
-      infinite = infinite || !(fabsf(r[0][h]) + fabsf(r[1][h]) + fabsf(r[2][h]) < kBwdFinite);
+      infinite = infinite || !(fabsf(r[0][h]) + fabsf(r[1][h]) + fabsf(r[2][h]) < kBwdFinite) ||
+                 !(fabsf(racc[h]) < INFINITY);
     }
     pix.py = make_float2(py[0], py[1]);
     pix.T = make_float2(T[0], T[1]);
@@ -1761,7 +1763,8 @@ __global__ void __launch_bounds__(128, FEW ? kFewTileBlocks : 8) k_backward_exac
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) whi = max(whi, __shfl_xor_sync(kFull, whi, o));
   if (lane == 0) s_hi[warp] = whi;
-  const bool finite_pixels = !__syncthreads_or(infinite);
+  // with the batches walked so far: racc keeps what an earlier one made of it
+  bool finite = !__syncthreads_or(infinite);
   int hi = s_hi[0];
   for (int w = 1; w < NW; ++w) hi = max(hi, s_hi[w]);
   const uint32_t red_word = 4u * (lane & 7u) + (lane >> 3);
@@ -1832,7 +1835,7 @@ __global__ void __launch_bounds__(128, FEW ? kFewTileBlocks : 8) k_backward_exac
         stage(k, q0, q1, q2, b.fmask[bhi - k]);
       }
     }
-    const bool finite = !__syncthreads_or(infinite) && finite_pixels;
+    finite = !__syncthreads_or(infinite) && finite;
     uint32_t nlist = 0;
     for (int base = 0; base < cnt; base += 32) {
       const int j = base + (int)lane;
