@@ -437,8 +437,8 @@ int sky_get_stage_times(void* ctx, double* ms, uint32_t n, uint64_t* steps);
  * Stable LSD radix sort of (u32 key, u32 value) pairs on the low key_bits
  * bits, replacing get_sorter(...).sort (src/sort/sort.ts:260-370,
  * radix_sort.wgsl:55-519).  All pointers are device pointers; stream is a
- * cudaStream_t (NULL = legacy default stream).  Input and output arrays must
- * not overlap.  Scratch is allocated and cached by the library per device.  */
+ * cudaStream_t (NULL = legacy default stream).  The arrays may start at any
+ * 4-byte boundary; input and output arrays must not overlap.  Scratch is allocated and cached by the library per device.  */
 int sky_sort_pairs(const uint32_t* keys_in, const uint32_t* vals_in, uint32_t* keys_out,
                    uint32_t* vals_out, uint32_t n, uint32_t key_bits, void* stream);
 

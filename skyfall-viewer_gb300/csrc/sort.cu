@@ -81,12 +81,14 @@ k_sort_hist(const uint32_t* __restrict__ keys, SortSegment seg, int passes, int 
     const uint32_t N = min(128u, n - base);  // valid keys of the chunk (a prefix)
     const uint32_t nvalid = idx >= n ? 0u : min(4u, n - idx);
     uint32_t k[4];
-    if (nvalid == 4u && ((begin + idx) & 3u) == 0u) {
-      const uint4 q = *reinterpret_cast<const uint4*>(keys + begin + idx);
+    // (by the address: a caller's array may start at any element of another)
+    const uint32_t* at = keys + begin + idx;
+    if (nvalid == 4u && (reinterpret_cast<uintptr_t>(at) & 15u) == 0u) {
+      const uint4 q = *reinterpret_cast<const uint4*>(at);
       k[0] = q.x; k[1] = q.y; k[2] = q.z; k[3] = q.w;
     } else {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) k[j] = (uint32_t)j < nvalid ? keys[begin + idx + j] : 0u;
+      for (int j = 0; j < 4; ++j) k[j] = (uint32_t)j < nvalid ? at[j] : 0u;
     }
     for (int p = digit_lo; p < passes; ++p) {
       const uint32_t dm = digit_mask(key_bits, p);
