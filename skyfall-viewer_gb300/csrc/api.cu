@@ -1968,7 +1968,7 @@ int sky_sort_pairs(const uint32_t* keys_in, const uint32_t* vals_in, uint32_t* k
     if (sc.mem) {
       CK(cudaDeviceSynchronize());
       cudaFree(sc.mem);
-      sc.mem = nullptr;
+      sc = SortCache{};  // (all of it: the allocation below may fail)
     }
     const size_t bytes = sort_scratch_bytes(n) + 256;
     if (inject_alloc()) return fail(SKY_ERR_INJECTED, "injected allocation failure");
