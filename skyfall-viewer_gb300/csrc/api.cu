@@ -58,19 +58,21 @@ int fail(int code, const char* fmt, ...) {
 // Host-side fault injection for tests of the error paths: SKY_FAULT=alloc:N
 // makes the N-th device allocation (1-based, process wide) fail with
 // SKY_ERR_INJECTED; SKY_FAULT=launch:N makes the N-th pass (step, forward,
-// backward or render) fail before it launches anything; SKY_FAULT=lookback:N
-// makes the N-th radix sort of a pass (item or intersection sort) or of
-// sky_sort_pairs run its bounded look-back waits out (tile 0 withholds its
-// word, 64 polls; see sort.cu), so that the call reports SKY_ERR_TIMEOUT.
-// Read once, when the first counted event happens.
+// backward or render) fail before it launches anything; SKY_FAULT=copy:N makes
+// the N-th copy of a render that leaves in chunks fail before it is issued;
+// SKY_FAULT=lookback:N makes the N-th radix sort of a pass (item or
+// intersection sort) or of sky_sort_pairs run its bounded look-back waits out
+// (tile 0 withholds its word, 64 polls; see sort.cu), so that the call reports
+// SKY_ERR_TIMEOUT.  Read once, when the first counted event happens.
 struct FaultPlan {
-  long alloc_at = -1, launch_at = -1, lookback_at = -1;
-  long allocs = 0, launches = 0, sorts = 0;
+  long alloc_at = -1, launch_at = -1, copy_at = -1, lookback_at = -1;
+  long allocs = 0, launches = 0, copies = 0, sorts = 0;
   FaultPlan() {
     const char* f = getenv("SKY_FAULT");
     if (!f) return;
     if (!strncmp(f, "alloc:", 6)) alloc_at = atol(f + 6);
     if (!strncmp(f, "launch:", 7)) launch_at = atol(f + 7);
+    if (!strncmp(f, "copy:", 5)) copy_at = atol(f + 5);
     if (!strncmp(f, "lookback:", 9)) lookback_at = atol(f + 9);
   }
 };
@@ -88,6 +90,11 @@ bool inject_launch() {
   std::lock_guard<std::mutex> l(g_fault_mu);
   FaultPlan& p = faults();
   return p.launch_at > 0 && ++p.launches == p.launch_at;
+}
+bool inject_copy() {
+  std::lock_guard<std::mutex> l(g_fault_mu);
+  FaultPlan& p = faults();
+  return p.copy_at > 0 && ++p.copies == p.copy_at;
 }
 
 }  // namespace
@@ -478,6 +485,20 @@ void drop_graph(Context* c) {
   c->gvalid = false;
 }
 
+// Whether all of a host range (none: p null) is page-locked, by its two ends.
+bool page_locked(const void* p, uint64_t bytes) {
+  if (!p) return true;
+  for (const char* at : {(const char*)p, (const char*)p + bytes - 1}) {
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, at) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    if (a.type != cudaMemoryTypeHost) return false;
+  }
+  return true;
+}
+
 // The chunks of a render of these views into host memory, none where copying
 // behind the kernel costs no more: below 8 MB of image (40 us at the 193 GB/s of
 // the link), and in chunks of at least 2048 tiles, two waves of the forward's
@@ -485,14 +506,6 @@ void drop_graph(Context* c) {
 // and one copy, 3.99 in 8 chunks on one stream, 3.85 on two streams in turn,
 // 3.72 in 16.  Only into page-locked memory: a 4K view into pageable memory
 // takes 77 ms in chunks and 7.4 in one copy.
-bool page_locked(const void* p) {
-  if (!p) return true;
-  cudaPointerAttributes a{};
-  if (cudaPointerGetAttributes(&a, p) == cudaSuccess) return a.type == cudaMemoryTypeHost;
-  cudaGetLastError();
-  return false;
-}
-
 std::vector<Chunk> render_chunks(const StepParams& sp, uint64_t bytes_per_px) {
   std::vector<Chunk> out;
   const uint64_t bytes = (uint64_t)sp.num_pixels * bytes_per_px;
@@ -520,6 +533,27 @@ std::vector<Chunk> render_chunks(const StepParams& sp, uint64_t bytes_per_px) {
 struct RenderOut {
   float *rgba, *alpha;
 };
+
+// Copies the chunks of a pass that has been enqueued, each as soon as it is
+// rendered, and waits for them; copied: false where the pass has failed.
+int copy_chunks(Context* c, const std::vector<Chunk>& chunks, const RenderOut& out, bool& copied) {
+  CK(cudaEventSynchronize(c->ready));
+  if (c->h_st->error != 0u) return SKY_OK;
+  auto copy = [&](float* dst, const Buf& src, uint64_t first, uint64_t n) -> int {
+    if (!dst) return SKY_OK;
+    if (inject_copy()) return fail(SKY_ERR_INJECTED, "injected copy failure");
+    CK(cudaMemcpyAsync(dst + first, (const float*)src.p + first, n * 4, cudaMemcpyDeviceToHost, c->copy_stream));
+    return SKY_OK;
+  };
+  for (size_t k = 0; k < chunks.size(); ++k) {
+    CK(cudaStreamWaitEvent(c->copy_stream, c->chunk_done[k], 0));
+    TRY(copy(out.rgba, c->color, chunks[k].px * 4, chunks[k].npx * 4));
+    TRY(copy(out.alpha, c->alpha, chunks[k].px, chunks[k].npx));
+  }
+  CK(cudaStreamSynchronize(c->copy_stream));
+  copied = true;
+  return SKY_OK;
+}
 
 // Runs one pass over `nv` cameras.  mode: render / forward (+loss) /
 // backward (gradients out, no Adam) / train (Adam step).  out: a render's
@@ -709,8 +743,9 @@ int run_views(Context* c, const uint32_t* cams, uint32_t nv, Mode mode, SkyStepS
   cudaStream_t s = c->stream;
   uint64_t launches = 0, h2d = 0, d2h = 0;
   std::vector<Chunk> chunks;
-  if (out && page_locked(out->rgba) && page_locked(out->alpha))
-    chunks = render_chunks(sp, (out->rgba ? 16 : 0) + (out->alpha ? 4 : 0));
+  if (out) chunks = render_chunks(sp, (out->rgba ? 16 : 0) + (out->alpha ? 4 : 0));
+  if (!chunks.empty() && !(page_locked(out->rgba, pix_total * 16) && page_locked(out->alpha, pix_total * 4)))
+    chunks.clear();
   if (!chunks.empty() && !c->ready) {
     if (!c->copy_stream) CK(cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking));
     if (!c->chunk_stream) CK(cudaStreamCreateWithFlags(&c->chunk_stream, cudaStreamNonBlocking));
@@ -728,24 +763,18 @@ int run_views(Context* c, const uint32_t* cams, uint32_t nv, Mode mode, SkyStepS
     // read-back left the GPU idle for about 25 us)
     const bool sizing = !graph && (!c->sized || attempt > 0);
     if (!graph) {
-      TRY(enqueue(c, sh, sizing, false, chunks, launches, h2d, d2h));
-      if (!chunks.empty()) {
-        // the lists are final: copy each chunk as soon as it is rendered
-        CK(cudaEventSynchronize(c->ready));
-        if (c->h_st->error == 0u) {
-          for (size_t k = 0; k < chunks.size(); ++k) {
-            const Chunk& ch = chunks[k];
-            CK(cudaStreamWaitEvent(c->copy_stream, c->chunk_done[k], 0));
-            if (out->rgba)
-              CK(cudaMemcpyAsync(out->rgba + ch.px * 4, (const float*)c->color.p + ch.px * 4, ch.npx * 16,
-                                 cudaMemcpyDeviceToHost, c->copy_stream));
-            if (out->alpha)
-              CK(cudaMemcpyAsync(out->alpha + ch.px, (const float*)c->alpha.p + ch.px, ch.npx * 4,
-                                 cudaMemcpyDeviceToHost, c->copy_stream));
-          }
-          CK(cudaStreamSynchronize(c->copy_stream));
-          copied = true;
+      int rc = enqueue(c, sh, sizing, false, chunks, launches, h2d, d2h);
+      if (rc == SKY_OK && !chunks.empty()) rc = copy_chunks(c, chunks, *out, copied);
+      if (rc != SKY_OK) {
+        // nothing may go on writing the caller's memory, reading the images that
+        // the next pass writes (it does not wait for these streams), or reading
+        // the parameters in host memory
+        if (!chunks.empty()) {
+          cudaStreamSynchronize(c->copy_stream);
+          cudaStreamSynchronize(c->chunk_stream);
         }
+        cudaStreamSynchronize(s);
+        return rc;
       }
     } else {
       if (!c->gvalid || !c->gshape.same(sh)) {
