@@ -1703,8 +1703,6 @@ SKY_DEV void reduce_slots(float* red, int ns, int j, float px, const BwdSplat* r
 // 16k Gaussians 109 -> 92 us (128 deep without the prefetch: 100; 64 with it:
 // 96), 475 tiles of 100k 169 -> 146, 768 of 16k 121 -> 105; 1024 of 16k 110 ->
 // 112, 16 views of 1M at 1080p 6574 -> 7545.
-constexpr int kFewTileBlocks = 5;
-constexpr uint32_t kFewTiles = kFewTileBlocks * 152;  // 152 multiprocessors
 template <int BB, bool CNT = false, bool FEW = false>
 __global__ void __launch_bounds__(128, FEW ? kFewTileBlocks : 8) k_backward_exact2(DevBuffers b) {
   chain_wait();
@@ -2899,7 +2897,7 @@ void launch_backward(const DevBuffers& b, uint32_t max_tiles, uint32_t ts, uint3
       case 8: chain(k_backward_exact<8>, max_tiles, 64, 0, s, b); break;
       case 32: chain(k_backward_exact<32>, max_tiles, 1024, 0, s, b); break;
       default: {
-        const bool few = max_tiles <= kFewTiles;
+        const bool few = few_tiles(max_tiles, sm_count());
         if (count && (bb == 0 || bb == kBwdBatch16)) {
           chain(k_backward_exact2<kBwdBatch16, true>, max_tiles, 128, 0, s, b);
           break;

@@ -23,9 +23,16 @@ void launch_flatten_fill(const DevBuffers& b, uint32_t total, cudaStream_t s);
 // other values select the defaults.  Results do not depend on them.
 // Default backward depth for 16x16 tiles (few tiles: 128, k_backward_exact2).
 constexpr uint32_t kBwdBatch16 = 64;
-// count: the pair-counting variants (16x16 tiles at the default depths
-// only; other shapes launch the plain kernels and count nothing).
-// The forward of tiles [first, first + tiles) alone (no SSIM term).
+// The 16x16 backward's variant for few tiles: where all of them are resident at
+// once, at this many blocks per multiprocessor of the device.
+constexpr int kFewTileBlocks = 5;
+inline bool few_tiles(uint32_t tiles, int multiprocessors) {
+  return tiles <= (uint32_t)kFewTileBlocks * (uint32_t)multiprocessors;
+}
+// count: the pair-counting variants (16x16 tiles at the default depths only;
+// other shapes launch the plain kernels and count nothing).  Counting steps of
+// few tiles run the 64-deep backward too.
+// launch_forward_tiles: tiles [first, first + tiles) alone (no SSIM term).
 void launch_forward_tiles(const DevBuffers& b, uint32_t first, uint32_t tiles, uint32_t ts, uint32_t fb,
                           bool count, cudaStream_t s);
 void launch_forward(const DevBuffers& b, uint32_t max_tiles, uint32_t ts, uint32_t fb, bool ssim,
