@@ -14,6 +14,7 @@ constexpr uint32_t kValueMask = (1u << 30) - 1u;
 constexpr uint32_t kSpinLimit = 1u << 20;
 constexpr int kWarps = kSortThreads / 32;
 constexpr int kLookBack = 2;
+constexpr int kRunStarts = 16;
 
 __device__ __forceinline__ uint32_t ld_relaxed(const uint32_t* p) {
   uint32_t v;
@@ -248,10 +249,14 @@ k_onesweep(const uint32_t* keys_src, const uint32_t* vals_src, uint32_t* keys_ds
   // The lanes that hold the same digit, of each of the warp's rounds: a ballot
   // per digit bit, four where the upper ones do not vary (the item sorts'
   // depths).  match.any serialises over the distinct values of a round, about
-  // 30 of 32 random bytes: 16.7M random keys 156 -> 136 us per pass; emission
-  // keys, in runs of equal digits, 125 -> 124.  Bound by the half-rate ALU pipe
-  // that the ballots' selects run on (73 % busy without the look-back); three
-  // blocks per multiprocessor (80 registers): four at 64 take 145 us.
+  // 30 of 32 random bytes: 16.7M random keys 156 -> 136 us per pass.  Where the
+  // keys come in runs it has few of them and is the faster one: a warp takes it
+  // for its 16 rounds when the first has fewer than kRunStarts starts of runs.
+  // 10M keys in runs of 2 / 4 / 8 / 50 (4 passes): ballots 374 / 371 / 370 / 370
+  // us, match.any 345 / 308 / 296 / 292, random keys 383 either way of the test.
+  // Bound by the half-rate ALU pipe that the ballots' selects run on (73 % busy
+  // without the look-back); three blocks per multiprocessor (80 registers):
+  // four at 64 take 145 us.
   uint32_t rank[kSortItems / 2];  // two 16-bit ranks within the warp's digit per word
   auto rank_keys = [&](auto bits) {
 #pragma unroll
@@ -273,7 +278,25 @@ k_onesweep(const uint32_t* keys_src, const uint32_t* vals_src, uint32_t* keys_ds
       rank[k / 2] = k % 2 ? rank[k / 2] | (rk << 16) : rk;
     }
   };
-  if (vary & 0xF0u) rank_keys(Bits<8>{});
+  auto rank_runs = [&]() {
+#pragma unroll
+    for (int k = 0; k < kSortItems; ++k) {
+      const uint32_t idx = base + warp * (32 * kSortItems) + k * 32 + lane;
+      const uint32_t d = (key[k] >> shift) & dmask;
+      const uint32_t peers = __match_any_sync(0xFFFFFFFFu, idx < n ? d : (uint32_t)kRadix);
+      const uint32_t cnt = s_warp_hist[warp][d];
+      __syncwarp();
+      if (idx < n && (peers & lt) == 0) s_warp_hist[warp][d] = cnt + __popc(peers);
+      __syncwarp();
+      const uint32_t rk = cnt + __popc(peers & lt);
+      rank[k / 2] = k % 2 ? rank[k / 2] | (rk << 16) : rk;
+    }
+  };
+  const uint32_t d0 = (key[0] >> shift) & dmask;
+  const uint32_t prev = __shfl_up_sync(0xFFFFFFFFu, d0, 1);
+  const bool runs = __popc(__ballot_sync(0xFFFFFFFFu, d0 != prev)) < kRunStarts;  // (lane 0: its own)
+  if (runs) rank_runs();
+  else if (vary & 0xF0u) rank_keys(Bits<8>{});
   else rank_keys(Bits<4>{});
   // the values are needed after the look-back: loaded now, off its path
   uint32_t val[kSortItems];
