@@ -376,7 +376,8 @@ int sky_train(void* ctx, uint32_t iterations, uint32_t views_per_step, SkyStepSt
  * min(10, cameras) drawn by the context's seeded generator; per Gaussian a
  * u32 importance (error-pixel hits) and an f32 pruning score (hits x mean
  * L1 of the view).  Scores are kept for sky_densify / sky_prune_scored in
- * the same iteration (getMultiViewScores :2790-2798).
+ * the same iteration (getMultiViewScores :2790-2798).  The context keeps 4
+ * bytes per Gaussian and view of a batch of up to 64 views for them.
  * sky_densify: clone/split on the device; new Gaussians are appended after
  * the survivors with zero Adam moments; resets both statistics.
  * sky_prune_scored: the weighted prune; resets both statistics.          */

@@ -1008,8 +1008,7 @@ int scan_flags(Context* c, const uint32_t* flags, uint32_t* out, uint32_t n) {
   sb.counts = (uint32_t*)flags;
   sb.cumsum = out;
   sb.block_sums = bs.as<uint32_t>();
-  launch_scan(sb, n, false, c->stream);
-  c->launches += 3;
+  c->launches += launch_scan(sb, n, false, c->stream);
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(c->stream));
   return SKY_OK;

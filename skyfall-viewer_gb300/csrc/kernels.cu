@@ -1278,8 +1278,8 @@ __global__ void __launch_bounds__(kLossThreads) k_loss_final(DevBuffers b) {
 // Gaussian later).  A warp skips a splat whose alpha >= 1/255 box misses all
 // of its pixels or that lies beyond all of its pixels' last contributors.
 // Each batch's per-pair values are reduced over the warp by a fixed
-// reduce-scatter (12 shuffles for 9 values; column first, 10 shuffles, in
-// the 16x16 kernel), then over the warps in index order, and written per
+// reduce-scatter (12 shuffles for 9 values; through shared memory, four
+// entries at a time, in the 16x16 kernel), then over the warps in index order, and written per
 // intersection to partials[emission index] -- so every Gaussian's partials
 // are contiguous and the later per-Gaussian sum has a fixed order.
 // ---------------------------------------------------------------------------
@@ -2958,8 +2958,8 @@ int launch_geom_adam(const DevBuffers& b, uint32_t n, uint32_t views, bool train
     return 1;
   }
   launch_geom_adam_as<true>(b, n, s);
-  // (a persistent grid: on the steps that leave the SH planes alone the launch
-  // is a few empty blocks)
+  // (a persistent grid of at most 16 blocks per multiprocessor: on the steps
+  // that leave the SH planes alone they return at once)
   const uint64_t work = (uint64_t)((n + 4 * kShAdamThreads - 1) / (4 * kShAdamThreads)) * kShGroups;
   const uint32_t blocks = (uint32_t)std::min<uint64_t>(work, (uint64_t)sm_count() * 16);
   chain(k_sh_adam, blocks, kShAdamThreads, 0, s, b);
